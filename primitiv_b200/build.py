@@ -11,12 +11,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(PKG, "libprimitiv_b200.so")
+BINDING = os.path.join(PKG, "binding", "native.cc")
+NATIVE = os.path.join(PKG, "_native.so")   # CPython module over the library
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -84,6 +87,15 @@ def build(verbose=False, force=False, dev_knobs=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    headers = [os.path.join(os.path.dirname(PKG), "include", f) for f in ("primitiv_b200.h", "primitiv_b200_ops.h")]
+    if force or _stale(NATIVE, [BINDING, os.path.abspath(__file__)] + headers):
+        cmd = ["g++", "-O3", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall",
+               "-I" + sysconfig.get_paths()["include"], BINDING, "-o", NATIVE, "-L" + PKG, "-lprimitiv_b200",
+               "-Wl,-rpath,$ORIGIN"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError("g++ failed: " + BINDING)
     with open(stamp, "w") as f:
         f.write(" ".join(flags))
     return LIB

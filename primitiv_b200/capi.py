@@ -1,10 +1,15 @@
-"""ctypes binding of include/primitiv_b200.h.
+"""Python binding of include/primitiv_b200.h.
 
 Device memory and streams come from the caller (raw integer addresses, e.g.
 ``torch.Tensor.data_ptr()``); this module never allocates through torch and has
 no compute of its own.
+
+``lib()`` is the library through ctypes.  The entry points that a training step calls
+thousands of times go through ``_native.so`` (binding/native.cc) instead, which takes plain
+numbers and None only; ``Context.op`` tries it first.
 """
 import ctypes
+import functools
 import os
 
 MODE_FP32_3XTF32 = 0
@@ -135,6 +140,20 @@ def _check(code, what=""):
         raise B200Error(code, what)
 
 
+def _call_ctypes(handle, name, *args):
+    _check(getattr(lib(), name)(handle, *args), name)
+
+
+def _caller(handle):
+    """``op`` of one context: the native wrapper where there is one and the arguments are plain."""
+    lib()
+    try:
+        from . import _native
+    except ImportError as e:
+        raise ImportError("primitiv_b200/_native.so is not built (run `python -m primitiv_b200.build`): %s" % e) from e
+    return _native.caller(handle.value, functools.partial(_call_ctypes, handle), _check)
+
+
 class Context:
     """One b200_ctx (one GPU).  Mirrors the lifetime of a primitiv::devices::B200 object."""
 
@@ -142,9 +161,11 @@ class Context:
         self._h = _vp()
         _check(lib().b200_ctx_create(device_id, ctypes.byref(self._h)), "b200_ctx_create")
         self.device_id = device_id
+        self.op = _caller(self._h)
 
     def close(self):
         if self._h:
+            del self.op   # it holds the context's address
             lib().b200_ctx_destroy(self._h)
             self._h = _vp()
 
@@ -186,7 +207,7 @@ class Context:
         _check(lib().b200_operand_cache_enable(self._h, max_bytes), "operand_cache_enable")
 
     def operand_cache_invalidate(self, ptr=None, nbytes=0):
-        _check(lib().b200_operand_cache_invalidate(self._h, ptr, nbytes), "operand_cache_invalidate")
+        self.op("b200_operand_cache_invalidate", ptr, nbytes)
 
     def operand_cache_stats(self):
         arr = (_u64 * 4)()
@@ -253,17 +274,15 @@ class Context:
 
     # -- hot path (device pointers as ints) --
     def matmul_fw(self, mode, a, b, y, di, dj, dk, ba, bb, stream=None):
-        _check(lib().b200_matmul_fw(self._h, mode, a, b, y, di, dj, dk, ba, bb, stream), "matmul_fw")
+        self.op("b200_matmul_fw", mode, a, b, y, di, dj, dk, ba, bb, stream)
 
     def matmul_bw(self, mode, a, b, gy, ga, gb, di, dj, dk, ba, bb, stream=None):
-        _check(lib().b200_matmul_bw(self._h, mode, a, b, gy, ga, gb, di, dj, dk, ba, bb, stream),
-               "matmul_bw")
+        self.op("b200_matmul_bw", mode, a, b, gy, ga, gb, di, dj, dk, ba, bb, stream)
 
     def matmul_bw_ex(self, mode, a, b, gy, ga, gb, di, dj, dk, ba, bb, accumulate_a=True, accumulate_b=True,
                      stream=None):
         """matmul_bw with `+=` (True) or `=` (False) per gradient; ga / gb may be None to skip one."""
-        _check(lib().b200_matmul_bw_ex(self._h, mode, a, b, gy, ga, gb, di, dj, dk, ba, bb,
-                                       int(accumulate_a), int(accumulate_b), stream), "matmul_bw_ex")
+        self.op("b200_matmul_bw_ex", mode, a, b, gy, ga, gb, di, dj, dk, ba, bb, int(accumulate_a), int(accumulate_b), stream)
 
     def matmul_fw_host(self, mode, a, b, y, di, dj, dk, ba, bb):
         _check(lib().b200_matmul_fw_host(self._h, mode, a, b, y, di, dj, dk, ba, bb), "matmul_fw_host")
@@ -274,18 +293,17 @@ class Context:
 
     def matmul_fw_bw_host(self, mode, a, b, gy, y, ga, gb, di, dj, dk, ba, bb, accumulate_a=True, accumulate_b=True):
         """Forward and both gradients from host buffers in one pipelined pass (addresses as ints, None to skip)."""
-        _check(lib().b200_matmul_fw_bw_host(self._h, mode, a, b, gy, y, ga, gb, di, dj, dk, ba, bb,
-                                            int(accumulate_a), int(accumulate_b)), "matmul_fw_bw_host")
+        self.op("b200_matmul_fw_bw_host", mode, a, b, gy, y, ga, gb, di, dj, dk, ba, bb, int(accumulate_a), int(accumulate_b))
 
     def selftest_wait_timeout(self, stream=None):
         _check(lib().b200_selftest_wait_timeout(self._h, stream), "selftest_wait_timeout")
 
     def op(self, name, *args):
-        """Calls any other entry point by name (the elementwise / movement / reduction set)."""
-        _check(getattr(lib(), name)(self._h, *args), name)
+        """Calls any other entry point by name (the elementwise / movement / reduction set).  An open
+        context has the native form of this in its place."""
+        _call_ctypes(self._h, name, *args)
 
     def gemm(self, mode, trans_a, trans_b, A, B, C, m, n, k, groups=1, red=1,
              a_gs=0, a_rs=0, b_gs=0, b_rs=0, c_gs=0, accumulate=False, force_path=0, stream=None):
-        _check(lib().b200_gemm(self._h, mode, int(trans_a), int(trans_b), A, B, C, m, n, k, groups, red,
-                               a_gs, a_rs, b_gs, b_rs, c_gs, int(accumulate), force_path, stream),
-               "gemm")
+        self.op("b200_gemm", mode, int(trans_a), int(trans_b), A, B, C, m, n, k, groups, red,
+                a_gs, a_rs, b_gs, b_rs, c_gs, int(accumulate), force_path, stream)
