@@ -103,8 +103,11 @@ class StagingRing {
 
 namespace b200 {
 
-// Cache of packed operand planes (fp32 mode).  An entry maps a dense source range of the caller's
-// memory to the block that holds its three planes in the source's own layout.  Entries live
+// Cache of packed operand planes.  An entry maps a dense source range of the caller's memory to the
+// block that holds its planes in the source's own layout: line by line where the lines had to be padded
+// for TMA (line = elements of a source line), element for element otherwise (line = 0).  Entries of the
+// single-pass modes, which the caller has not opted into, never outlive the entry point that made them
+// (call_only); those of the fp32 mode live
 // while the cache is enabled (b200_operand_cache_enable) or while an entry point that uses an
 // operand more than once is running (scope > 0), and die when their source range is written
 // (b200_operand_cache_invalidate), returned to the pool, or evicted to stay under the byte cap.
@@ -115,6 +118,9 @@ struct PlaneCache {
     void *block;
     std::size_t block_bytes;
     std::uint64_t stamp;
+    int kind;              // PlaneKind (pack.h)
+    std::uint32_t line;
+    bool call_only;
   };
   std::vector<Entry> entries;
   std::size_t bytes = 0, cap = 0;   // cap == 0: not enabled by the caller
@@ -214,14 +220,29 @@ struct GemmArgs {
   int accumulate;
 };
 
+// Tiny and thin products are bound by latency or by the large operand's bytes: even in TF32 mode they are
+// given fp32-grade arithmetic, which costs next to nothing there.
+inline bool tiny_or_thin(const GemmArgs &g) {
+  const double macs = static_cast<double>(g.m) * g.n * g.k * g.groups * g.red;
+  return macs < 2097152.0 || g.n < 16u || (g.m < 32u && macs < 67108864.0);
+}
+
 // CUDA-core path: any shape, any alignment.
 int gemm_simt(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // CUDA-core kernels for products with one tiny extent against large ones (gemm_skinny.cu).
 bool gemm_skinny_eligible(const GemmArgs &g);
 int gemm_skinny(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
+// mma.sync path: any shape, any alignment, operands read where they lie (gemm_mma.cuh).
+int gemm_mma(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // tcgen05 path.  tc_eligible() says whether the operands meet TMA's alignment rules.
 bool gemm_tc_eligible(const b200_ctx *ctx, const GemmArgs &g);
 int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
+// Whether it needs no pass over the operands first.
+bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g);
+// Microseconds either path would take on an otherwise idle GPU, the launch included: for choosing
+// between them.  1e30: not eligible.
+double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g);
+double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g);
 // Checks (and re-arms) the guard bands of every pool block; see b200_pool_check_guards.
 int pool_check_guards(b200_ctx *ctx, cudaStream_t stream, std::uint64_t *damaged, void **first, int *side);
 // Streams L2-resident data into every SM's shared memory and reports the rate; see b200_measure_l2_ingest.
@@ -234,12 +255,15 @@ int gemm_3xtf32_noalloc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // Operand-plane cache (see PlaneCache).  drop_range forgets every entry whose source overlaps
 // [ptr, ptr + bytes) (everything when ptr is null) and returns its block to the pool.
 void plane_cache_drop_range(b200_ctx *ctx, const void *ptr, std::size_t bytes);
+void plane_cache_drop_call_only(b200_ctx *ctx);
 // Brackets an entry point that hands the same operand to several products.
 struct PlaneScope {
   b200_ctx *ctx;
   explicit PlaneScope(b200_ctx *c) : ctx(c) { ++ctx->planes.scope; }
   ~PlaneScope() {
-    if (--ctx->planes.scope == 0 && ctx->planes.cap == 0) plane_cache_drop_range(ctx, nullptr, 0);
+    if (--ctx->planes.scope != 0) return;
+    if (ctx->planes.cap == 0) plane_cache_drop_range(ctx, nullptr, 0);
+    else plane_cache_drop_call_only(ctx);
   }
 };
 

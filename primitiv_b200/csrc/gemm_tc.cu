@@ -61,6 +61,7 @@
 // waits, frees TMEM and returns.
 #include <cuda_fp16.h>
 
+#include <cstdio>
 #include <cstdlib>
 #include <cstring>
 
@@ -447,25 +448,27 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
 // must assume they alias) and the epilogue would pay one memory latency per column.
 // kWide = old values in flight per thread: 8 where registers are tight (the chunked kernel holds
 // a whole tile row in registers), 32 elsewhere.
-template <uint32_t kWide, bool kAccumulate, typename T>
+// kWhole: all 32 columns exist.  With a bounds check per column the compiler branched round every
+// store, and a 128 x 256 tile took 4.5 us to write where its stores alone need less than one.
+template <uint32_t kWide, bool kAccumulate, bool kWhole, typename T>
 __device__ __forceinline__ void store_cols_as(T *C, unsigned long long base, uint32_t m, uint32_t n,
                                               uint32_t col0, const float (&x)[32]) {
   T *q = C + base + static_cast<unsigned long long>(col0) * m;
-  const uint32_t left = n - col0;  // caller guarantees col0 < n
+  const uint32_t left = kWhole ? 32u : n - col0;  // caller guarantees col0 < n
 #pragma unroll
   for (uint32_t h = 0; h < 32u; h += kWide) {  // kWide loads in flight per thread, then kWide stores
     float old[kWide];
 #pragma unroll
     for (uint32_t j = 0; j < kWide; ++j) {
       old[j] = 0.f;
-      if (kAccumulate && h + j < left) {
+      if (kAccumulate && (kWhole || h + j < left)) {
         if constexpr (sizeof(T) == 2) old[j] = __half2float(q[static_cast<unsigned long long>(h + j) * m]);
         else old[j] = q[static_cast<unsigned long long>(h + j) * m];
       }
     }
 #pragma unroll
     for (uint32_t j = 0; j < kWide; ++j) {
-      if (h + j < left) {
+      if (kWhole || h + j < left) {
         const float v = x[h + j] + old[j];
         if constexpr (sizeof(T) == 2) q[static_cast<unsigned long long>(h + j) * m] = __float2half_rn(v);
         else q[static_cast<unsigned long long>(h + j) * m] = v;
@@ -479,8 +482,13 @@ __device__ __forceinline__ void store_cols_as(T *C, unsigned long long base, uin
 template <uint32_t kWide, typename T>
 __device__ __forceinline__ void store_cols(T *C, unsigned long long base, uint32_t m, uint32_t n,
                                            uint32_t col0, const float (&x)[32], bool accumulate) {
-  if (accumulate) store_cols_as<kWide, true>(C, base, m, n, col0, x);
-  else store_cols_as<kWide, false>(C, base, m, n, col0, x);
+  if (n - col0 >= 32u) {
+    if (accumulate) store_cols_as<kWide, true, true>(C, base, m, n, col0, x);
+    else store_cols_as<kWide, false, true>(C, base, m, n, col0, x);
+  } else {
+    if (accumulate) store_cols_as<kWide, true, false>(C, base, m, n, col0, x);
+    else store_cols_as<kWide, false, false>(C, base, m, n, col0, x);
+  }
 }
 
 // Tile order.  Tiles of one group (one output matrix) are walked in bands of kBandTilesM
@@ -550,6 +558,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   const uint32_t first_tile = blockIdx.x / kCtas;   // tiles are dealt to CTAs (kCtas == 1) or to pairs
   const uint32_t tile_step = gridDim.x / kCtas;
 
+  if (threadIdx.x == 32u * 2u) {
+    // the tensor maps are parameters: their fetch need not wait for the grid in front
+    constexpr uint32_t kMaps = kMix ? 0xf5u : kPasses == 3 ? 0x0fu : 0x05u;   // those this kind encodes, in the order they lie
+    for (uint32_t i = 0; i < 8u; ++i)
+      if (kMaps >> i & 1u)
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(&p.mapA[0] + i)) : "memory");
+  }
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (uint32_t s = 0; s < p.stages; ++s) {
@@ -1035,14 +1050,90 @@ bool gemm_tc_eligible(const b200_ctx *ctx, const GemmArgs &g) {
   if (!stride_pattern(g.a_gs, g.a_rs, g.groups, g.red, &sta, &nba, &gm, &rm)) return false;
   if (!stride_pattern(g.b_gs, g.b_rs, g.groups, g.red, &stb, &nbb, &gm, &rm)) return false;
   if (g.mode == B200_MODE_FP16) {
-    // half operands are never repacked: they must satisfy TMA's alignment rules as they lie
+    // half operands are read where they lie, or with their lines padded, which takes dense matrices
     const uint64_t lda = g.trans_a ? g.k : g.m, ldb = g.trans_b ? g.n : g.k;
-    return direct_ok(g.A, lda, sta, nba, 2) && direct_ok(g.B, ldb, stb, nbb, 2);
+    return (direct_ok(g.A, lda, sta, nba, 2) || nba == 1 || sta == static_cast<uint64_t>(g.m) * g.k) &&
+           (direct_ok(g.B, ldb, stb, nbb, 2) || nbb == 1 || stb == static_cast<uint64_t>(g.n) * g.k);
   }
   return true;  // fp32: whatever is not directly loadable goes through the packing pre-pass
 }
 
 namespace {
+
+// ---- choice of tile and split ----
+//
+// What a launch takes is estimated from what was measured on 57 products of 256^3 to 2048^3 and
+// their flat, tall and batched relatives in all four kinds, each with every tile and split:
+//   - an SM takes operand tiles in at 110 GB/s (16-bit kinds) or 90 GB/s (32-bit kinds), or the tensor
+//     core works through them at bn / 2 clocks per instruction, whichever is slower;
+//   - writing a tile takes 12.5 ns per column, hidden behind the next tile's main loop unless that is
+//     shorter, except for the last;
+//   - a tile costs 1 us besides (its pipeline fills and drains), a CTA pair 1 us per launch, a split 2.5 us and
+//     the partial tiles' way through L2.
+// The choice this gives is within 1 % of the best one on average over those products.  Against the rule
+// before it (256-column pair tiles wherever they fit, splits only below half a wave): 1024^3 halves 10.4 ->
+// 7.2 us, 1024^3 TF32 17.4 -> 12.9, 9 x 512 x 384 x 1024 TF32 20.6 -> 13.6, 8 x 256 x 1024 x 256 fp32 12.2 -> 9.5.
+// (Pairs of 128 columns were measured too: never better than single CTAs of 128.)
+struct TileChoice {
+  uint32_t ctas, bn, splits;
+  double us;   // estimate without the launch itself
+};
+
+struct TileCost {
+  uint32_t planes_bytes;   // operand bytes per row of a 128-byte k-block (all planes)
+  uint32_t mma_per_kblock; // tensor-core instructions per k-block
+  double bytes_per_us;
+};
+
+TileChoice choose_tile(const b200_ctx *ctx, const GemmArgs &g, const TileCost &cost, uint32_t kblocks, uint32_t kblocks_per_stage,
+                       bool may_split) {
+  const double clocks_per_us = 1850.0;
+  static const struct { uint32_t ctas, bn; } kShapes[] = {{2, 256}, {1, 256}, {1, 128}, {1, 64}};
+  TileChoice best{1, 64, 1, 1e30};
+  for (const auto &sh : kShapes) {
+    if (sh.bn > 64u && sh.bn / 2u >= g.n) continue;   // half the columns or more would be padding
+    if (sh.ctas == 2u && (g.m <= kBM || ctx->sm_count < 2 || ctx->pair_policy == 1)) continue;
+    const uint32_t rows = kBM * sh.ctas;
+    const double tiles = static_cast<double>((g.m + rows - 1) / rows) * ((g.n + sh.bn - 1) / sh.bn) * g.groups;
+    const double units = ctx->sm_count / static_cast<int>(sh.ctas);
+    const double load = (kBM + sh.bn / sh.ctas) * static_cast<double>(cost.planes_bytes) / cost.bytes_per_us;
+    const double mma = cost.mma_per_kblock * (sh.bn / 2.0) / clocks_per_us;
+    const double per_kblock = load > mma ? load : mma;
+    const uint32_t stages_k = (kblocks + kblocks_per_stage - 1) / kblocks_per_stage;
+    // (a split is at least two pipeline stages, and never more work items than one wave)
+    for (uint32_t s = 1; s <= 64u && (s == 1u || (may_split && s * 2u <= stages_k && tiles * s <= units)); s += s < 4u ? 1u : s / 4u) {
+      const double kb = static_cast<double>((stages_k + s - 1) / s) * kblocks_per_stage * g.red;
+      const double waves = static_cast<double>(static_cast<uint64_t>((tiles * s + units - 1) / units));
+      const double main = kb * per_kblock + 1.0, write = 0.0125 * sh.bn;
+      double us = waves * (main > write ? main : write) + (main > write ? write : main) + (sh.ctas == 2u ? 1.0 : 0.0);
+      if (s > 1u) us += 2.5 + static_cast<double>(g.m) * g.n * g.groups * (s + 1u) * 4.0 / 4e6;
+      if (us < best.us) best = {sh.ctas, sh.bn, s, us};
+    }
+  }
+  return best;
+}
+
+TileCost tile_cost(int mode, bool mix) {
+  const bool f16 = mode == B200_MODE_FP16 || mode == B200_MODE_FP32_3XFP16;
+  const uint32_t passes = mode == B200_MODE_FP32_3XTF32 || mode == B200_MODE_FP32_3XFP16 ? 3u : 1u;
+  return {passes == 3u ? 256u : 128u, mix ? 8u : 4u * passes, f16 ? 110e3 : 90e3};
+}
+
+// What fetching one operand costs before the product: nothing where TMA reads it in place or its planes are
+// cached; else a launch and the bytes it moves, at the rates of the kernels in pack.cu.
+double pack_us(const b200_ctx *ctx, const OperandView &v, int mode, bool is_b, uint32_t m) {
+  const double elems = static_cast<double>(v.mn) * v.k * (v.nbatch ? v.nbatch : 1u);
+  if (mode == B200_MODE_FP16 || mode == B200_MODE_TF32) {
+    if (direct_ok(v.ptr, v.ld, v.batch_stride, v.nbatch, elem_bytes(mode))) return 0.0;
+    if (flat_cached(ctx, v, mode == B200_MODE_FP16 ? kPlanesHalf : kPlanesTf32)) return 0.0;
+    return 2.0 + elems * 2.0 * elem_bytes(mode) / 4e6;
+  }
+  if (mode == B200_MODE_FP32_3XFP16) return (v.mn_major ? 6.0 : 2.5) + elems * 8.0 / 4e6;
+  if (is_b && v.mn_major && m > 1536u) return 2.0 + elems * 12.0 / 4e6;   // transposed
+  if (flat_cached(ctx, v, kPlanesMix)) return 0.0;
+  // (with the cache on, planes serve two products of a step)
+  return (ctx->planes.cap ? 0.6 : 1.0) * (2.0 + elems * 12.0 / 5e6);
+}
 
 // Shared body of gemm_tc and of the allocation-free entry point.  With
 // fixed_scratch == nullptr the packing planes come from the context's pool; otherwise
@@ -1065,16 +1156,23 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   p.bk = 128u / eb;                       // 128 bytes of k per stage
   const uint32_t umma_k = 32u / eb;       // 8 (tf32) or 16 (fp16)
   const uint32_t chunk = 128u / eb;       // mn elements per 128-byte swizzle row
-  p.bn = g.n > 128 ? 256u : (g.n > 64 ? 128u : 64u);
   p.m = g.m;
   p.n = g.n;
   p.k = g.k;
   p.kblocks = (g.k + p.bk - 1) / p.bk;
   p.red = g.red;
   p.groups = g.groups;
-  // A pair of CTAs per 256-row tile when the problem has the rows and columns for it
-  // (each CTA then stages bn/2 >= 64 rows of B) and the context allows it.
-  const uint32_t ctas = (ctx->pair_policy != 1 && g.m > kBM && p.bn >= 128u && ctx->sm_count >= 2) ? 2u : 1u;
+  static const char *sp = kDevKnobs ? std::getenv("PRIMITIV_B200_TC_SPLIT") : nullptr;  // 0 = never split
+  const bool may_split = !fixed_scratch && ctx->split_policy != 1 && !(sp && std::atoi(sp) == 0);
+  TileChoice tile = choose_tile(ctx, g, tile_cost(g.mode, mix), p.kblocks, passes == 1 ? 2u : 1u, may_split);
+  if (ctx->pair_policy >= 2 && g.m > kBM && g.n >= 128u && ctx->sm_count >= 2) tile = {2u, g.n > 128u ? 256u : 128u, 1u, 0.0};   // (tests)
+  if (kDevKnobs) {
+    int c = 0, n = 0, k = 0;
+    const char *e = std::getenv("PRIMITIV_B200_TC_CFG");
+    if (e && std::sscanf(e, "%d,%d,%d", &c, &n, &k) == 3) tile = {static_cast<uint32_t>(c), static_cast<uint32_t>(n), static_cast<uint32_t>(k), 0.0};
+  }
+  p.bn = tile.bn;
+  const uint32_t ctas = tile.ctas;
   const uint32_t tile_m = kBM * ctas;
   p.tiles_m = (g.m + tile_m - 1) / tile_m;
   // Half storage, pairs: a 256 x 512 tile per pair (see gemm_tc_kernel, kWide) for long contractions
@@ -1120,11 +1218,11 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   bool b_hybrid = false;
   OperandView vb8;
   if (mix) {
-    // An operand that is dense and 32-byte aligned in every stride is packed "flat": the three
-    // planes repeat the caller's layout element for element (the kernel reads either
-    // major-ness), the pre-pass is purely elementwise, and the planes can serve every later
-    // use of the same array, whichever side of whichever product it is on: they go through the
-    // context's plane cache.  Anything else is repacked K-major into scratch for this launch.
+    // A dense operand is packed "flat": the three planes repeat the caller's layout, element for
+    // element or with its lines padded to what TMA wants (the kernel reads either major-ness), and the
+    // planes can serve every later use of the same array, whichever side of whichever product it is
+    // on: they go through the context's plane cache.  Anything else is repacked K-major into
+    // scratch for this launch.
     OperandView *views[2] = {&va, &vb};
     const void **outs[2] = {a_mix, b_mix};
     bool *flat[2] = {&a_flat, &b_flat};
@@ -1138,12 +1236,14 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
       // meet near m = 1800.  That is the weight gradient of a layer, gW = gZ . H^T over a large
       // minibatch, whose H was split flat for the forward product.)
       const bool b_mn = o == 1 && views[o]->mn_major;
-      const bool flat_possible = !fixed_scratch && ctx->correction_policy == 0 && mix_flat_ok(*views[o]);
-      const bool cached = flat_possible && b_mn && mix_flat_cached(ctx, *views[o]);
+      const bool flat_possible = !fixed_scratch && ctx->correction_policy == 0 && flat_ok(*views[o]);
+      const bool cached = flat_possible && b_mn && flat_cached(ctx, *views[o], kPlanesMix);
+      // (padding lines is also much cheaper than the transposing pre-pass of ragged extents)
+      const bool ragged = flat_possible && !flat_exact(*views[o]);
       // (a small B as well, whatever m: its transposing pre-pass would be one more launch in a chain of
       // few-microsecond kernels, more than a fifth of such a product's main loop)
       const bool small_b = static_cast<uint64_t>(views[o]->mn) * views[o]->k * (views[o]->nbatch ? views[o]->nbatch : 1u) < (1ull << 20);
-      *flat[o] = flat_possible && (!b_mn || ((g.m <= 1536u || small_b) && cached));
+      *flat[o] = flat_possible && (!b_mn || ((g.m <= 1536u || small_b) && (cached || ragged)));
       // Only the TF32 plane of an MN-major B is slow to read; its bf16 planes are not.  With the flat
       // planes already cached, the transposing pre-pass therefore writes the TF32 plane alone (8
       // instead of 12 bytes per element) and the correction passes read the cached bf16 planes.
@@ -1164,16 +1264,16 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
     }
     for (int o = 0; o < 2; ++o) {
       if (*flat[o]) {
-        const int rc = mix_flat_planes(ctx, stream, *views[o], outs[o], &flat_blocks[o]);
+        const int rc = flat_planes(ctx, stream, *views[o], kPlanesMix, outs[o], &flat_blocks[o]);
         if (rc != B200_OK) {
           release();
           return rc;
         }
       } else if (o == 1 && b_hybrid) {
-        vb8 = vb;   // the caller's layout: what the cached bf16 planes repeat
-        const void *flat_planes[3];
+        vb8 = vb;   // the caller's layout: what the cached planes repeat
+        const void *cached_planes[3];
         void *unused = nullptr;
-        const int rc = mix_flat_planes(ctx, stream, vb, flat_planes, &unused);   // a cache hit: nothing is packed
+        const int rc = flat_planes(ctx, stream, vb8, kPlanesMix, cached_planes, &unused);   // a cache hit: nothing is packed
         if (rc != B200_OK || unused) {
           if (unused) ctx->pool.free(unused);
           release();
@@ -1181,8 +1281,8 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
         }
         pack_mix(ctx, stream, vb, cursor, lay[o], outs[o], /*hi_only=*/true);
         cursor += lay[o].hi_elems;
-        b_mix[1] = flat_planes[1];
-        b_mix[2] = flat_planes[2];
+        b_mix[1] = cached_planes[1];
+        b_mix[2] = cached_planes[2];
       } else {
         pack_mix(ctx, stream, *views[o], cursor, lay[o], outs[o]);
         cursor += lay[o].floats();
@@ -1201,7 +1301,22 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
     pack_f16(ctx, stream, vb, lb, base + la.bytes(), b_src, &p.scale_b);
     p.scale_a_gs = (!la.shared && p.a_gmul) ? g.m : 0u;
     p.scale_b_gs = (!lb.shared && p.b_gmul) ? g.n : 0u;
-  } else if (!f16) {
+  } else if (f16) {
+    // lines that TMA cannot address are padded
+    OperandView *views[2] = {&va, &vb};
+    const void **srcs[2] = {a_src, b_src};
+    for (int o = 0; o < 2; ++o) {
+      const OperandView &v = *views[o];
+      if (direct_ok(v.ptr, v.ld, v.batch_stride, v.nbatch, 2)) continue;
+      const void *planes[3];
+      const int rc = fixed_scratch ? B200_ERR_INVALID_ARG : flat_planes(ctx, stream, *views[o], kPlanesHalf, planes, &flat_blocks[o]);
+      if (rc != B200_OK) {
+        release();
+        return rc;
+      }
+      srcs[o][0] = planes[0];
+    }
+  } else {
     // 3xTF32 always repacks, even operands the tensor core could read where they lie (it
     // truncates fp32 words to TF32, so the caller's array could serve as the hi plane and only
     // lo = rn(x - trunc(x)) be written).  That was tried: the pre-pass got a third cheaper, but
@@ -1210,7 +1325,7 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
     OperandView *views[2] = {&va, &vb};
     const void **srcs[2] = {a_src, b_src};
     Tf32Planes lay[2];
-    bool pack[2];
+    bool pack[2], pad[2];
     uint64_t total = 0;
     const uint64_t planes = passes == 3 ? 2 : 1;
     for (int o = 0; o < 2; ++o) {
@@ -1223,7 +1338,9 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
                           static_cast<uint64_t>(v.mn) * v.k * (v.nbatch ? v.nbatch : 1u) >= (1ull << 22);
       pack[o] = passes == 3 || slow_b || !direct_ok(v.ptr, v.ld, v.batch_stride, v.nbatch, 4);
       lay[o] = tf32_planes(v);
-      if (pack[o]) total += planes * lay[o].plane_elems;
+      // (what only lacks alignment keeps its layout, with padded lines)
+      pad[o] = pack[o] && passes == 1 && !slow_b && !fixed_scratch && flat_ok(v);
+      if (pack[o] && !pad[o]) total += planes * lay[o].plane_elems;
     }
     float *cursor = nullptr;
     if (total && fixed_scratch) {
@@ -1236,6 +1353,16 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
     }
     for (int o = 0; o < 2; ++o) {
       if (!pack[o]) continue;
+      if (pad[o]) {
+        const void *planes[3];
+        const int rc = flat_planes(ctx, stream, *views[o], kPlanesTf32, planes, &flat_blocks[o]);
+        if (rc != B200_OK) {
+          release();
+          return rc;
+        }
+        srcs[o][0] = planes[0];
+        continue;
+      }
       pack_tf32(ctx, stream, *views[o], passes == 3, cursor, lay[o], srcs[o]);
       cursor += planes * lay[o].plane_elems;
     }
@@ -1264,24 +1391,13 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   }
   p.stage_bytes = p.subs * p.sub_bytes;
   p.kblocks = (g.k + p.bk * p.subs - 1) / (p.bk * p.subs);  // pipeline-stage iterations along k
-  // Split-K: with fewer tiles than half the CTAs (or pairs) and a long contraction, slices of k go
-  // to the idle ones (at least four pipeline stages each) and splitk_reduce_kernel adds them up.
+  // Split-K: slices of k go to CTAs (or pairs) that the tiles alone would leave idle, and splitk_reduce_kernel adds them up.
   uint32_t splits = 1;
   void *partial = nullptr;
-  {
-    const uint64_t units = static_cast<uint64_t>(ctx->sm_count) / ctas;
-    static const char *sp = kDevKnobs ? std::getenv("PRIMITIV_B200_TC_SPLIT") : nullptr;  // 0 = never split
-    const bool allow = !(sp && std::atoi(sp) == 0) && ctx->split_policy != 1 && !wide;   // (the wide epilogue stores halves only)
-    if (!fixed_scratch && allow && total_tiles * 2 <= units && p.kblocks >= 16u) {
-      uint64_t want = units / total_tiles;
-      if (want > p.kblocks / 4u) want = p.kblocks / 4u;
-      if (want > 64u) want = 64u;
-      if (want >= 2u) {
-        const uint32_t per = (p.kblocks + static_cast<uint32_t>(want) - 1u) / static_cast<uint32_t>(want);
-        splits = (p.kblocks + per - 1u) / per;  // no empty slices
-        p.kblocks = per;
-      }
-    }
+  if (tile.splits > 1u && !wide) {   // (the wide epilogue stores halves only)
+    const uint32_t per = (p.kblocks + tile.splits - 1u) / tile.splits;
+    splits = (p.kblocks + per - 1u) / per;  // no empty slices
+    p.kblocks = per;
   }
   p.splits = splits;
   p.groups = g.groups * splits;
@@ -1540,6 +1656,37 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
 }
 
 }  // namespace
+
+namespace {
+void operand_views(const GemmArgs &g, OperandView *a, OperandView *b) {
+  uint32_t gm, rm;
+  *a = {g.A, g.m, g.k, !g.trans_a, g.trans_a ? g.k : g.m, 0, 1};
+  stride_pattern(g.a_gs, g.a_rs, g.groups, g.red, &a->batch_stride, &a->nbatch, &gm, &rm);
+  *b = {g.B, g.n, g.k, g.trans_b != 0, g.trans_b ? g.n : g.k, 0, 1};
+  stride_pattern(g.b_gs, g.b_rs, g.groups, g.red, &b->batch_stride, &b->nbatch, &gm, &rm);
+}
+}  // namespace
+
+bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g) {
+  if (g.mode != B200_MODE_FP16 && g.mode != B200_MODE_TF32) return false;
+  if (!gemm_tc_eligible(ctx, g)) return false;
+  OperandView a, b;
+  operand_views(g, &a, &b);
+  const int eb = elem_bytes(g.mode);
+  return direct_ok(a.ptr, a.ld, a.batch_stride, a.nbatch, eb) && direct_ok(b.ptr, b.ld, b.batch_stride, b.nbatch, eb);
+}
+
+double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g) {
+  if (!gemm_tc_eligible(ctx, g) || (g.mode == B200_MODE_TF32 && tiny_or_thin(g))) return 1e30;
+  OperandView a, b;
+  operand_views(g, &a, &b);
+  const bool half = g.mode == B200_MODE_FP16 || g.mode == B200_MODE_FP32_3XFP16;
+  const bool one = g.mode == B200_MODE_FP16 || g.mode == B200_MODE_TF32;
+  const bool mix = g.mode == B200_MODE_FP32_3XTF32 && ctx->correction_policy != 1;
+  const uint32_t bk = half ? 64u : 32u;
+  const TileChoice t = choose_tile(ctx, g, tile_cost(g.mode, mix), (g.k + bk - 1) / bk, one ? 2u : 1u, ctx->split_policy != 1);
+  return 3.0 + t.us + pack_us(ctx, a, g.mode, false, g.m) + pack_us(ctx, b, g.mode, true, g.m);
+}
 
 int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream) {
   return gemm_tc_run(ctx, g, stream, nullptr, 0);

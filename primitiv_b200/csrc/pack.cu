@@ -521,6 +521,47 @@ __global__ void __launch_bounds__(256) pack_mix_kernel(const float *__restrict__
   }
 }
 
+// Any dense source, line by line, lines padded to `pad` elements (a multiple of 8) in the planes and the
+// padding left as it is (TMA is given the true extents).  1 << shift lanes walk a line, two elements a
+// lane and step, four steps in flight.  Bound by memory; what it replaces for ragged sizes transposed every
+// operand through 32 x 32 tiles in shared memory, for one use.
+template <int kKind, typename T>
+__global__ void __launch_bounds__(256) pad_lines_kernel(const T *__restrict__ src, void *__restrict__ p0, void *__restrict__ p1,
+                                                        void *__restrict__ p2, uint32_t line, uint32_t pad,
+                                                        unsigned long long lines, uint32_t shift) {
+  pdl_enter();
+  const uint32_t lanes = 1u << shift, lane = threadIdx.x & (lanes - 1u);
+  const unsigned long long step = (static_cast<unsigned long long>(gridDim.x) * 256u) >> shift;
+  for (unsigned long long l = (blockIdx.x * 256ull + threadIdx.x) >> shift; l < lines; l += step) {
+    const T *s = src + l * line;
+    const unsigned long long d = l * pad;
+    for (uint32_t e0 = lane * 2u; e0 < line; e0 += lanes * 8u) {
+      T x[4][2];
+#pragma unroll
+      for (uint32_t u = 0; u < 4u; ++u) {
+        const uint32_t e = e0 + u * lanes * 2u;
+        x[u][0] = e < line ? s[e] : T(0.f);
+        x[u][1] = e + 1u < line ? s[e + 1u] : T(0.f);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < 4u; ++u) {
+        const uint32_t e = e0 + u * lanes * 2u;
+        if (e >= line) break;
+        if constexpr (kKind == kPlanesHalf) {
+          reinterpret_cast<__half2 *>(p0)[(d + e) >> 1] = __halves2half2(x[u][0], x[u][1]);
+        } else {
+          const float2 h = make_float2(rn_tf32(x[u][0]), rn_tf32(x[u][1]));
+          reinterpret_cast<float2 *>(p0)[(d + e) >> 1] = h;
+          if constexpr (kKind == kPlanesMix) {
+            reinterpret_cast<uint32_t *>(p1)[(d + e) >> 1] = bf16_pair(x[u][0], x[u][1]);
+            reinterpret_cast<uint32_t *>(p2)[(d + e) >> 1] = bf16_pair(x[u][0] - h.x, x[u][1] - h.y);
+          }
+        }
+      }
+    }
+  }
+}
+
 }  // namespace
 
 Tf32Planes tf32_planes(const OperandView &v) {
@@ -626,14 +667,15 @@ void pack_mix(b200_ctx *ctx, cudaStream_t stream, OperandView &v, float *dst, co
   v.batch_stride = static_cast<uint64_t>(v.mn) * lay.kpad;
 }
 
-// ------------------------------ flat planes and their cache ------------------------------
+// ------------------------------ planes in the operand's layout, and their cache ------------------------------
 
-bool mix_flat_ok(const OperandView &v) {
-  if (reinterpret_cast<uintptr_t>(v.ptr) & 31u) return false;
+bool flat_ok(const OperandView &v) {
   const uint64_t inner = v.mn_major ? v.mn : v.k;
-  if (v.ld != inner || inner % 8u) return false;                                        // dense, 32-byte rows
-  if (v.nbatch > 1 && v.batch_stride != static_cast<uint64_t>(v.mn) * v.k) return false;  // matrices back to back
-  return true;
+  return v.ld == inner && (v.nbatch <= 1 || v.batch_stride == static_cast<uint64_t>(v.mn) * v.k);
+}
+
+bool flat_exact(const OperandView &v) {
+  return (reinterpret_cast<uintptr_t>(v.ptr) & 31u) == 0 && (v.mn_major ? v.mn : v.k) % 8u == 0;
 }
 
 void plane_cache_drop_range(b200_ctx *ctx, const void *ptr, std::size_t bytes) {
@@ -657,32 +699,87 @@ void plane_cache_drop_range(b200_ctx *ctx, const void *ptr, std::size_t bytes) {
   for (void *b : blocks) ctx->pool.free(b);   // stream-ordered reuse: queued products that read them run first
 }
 
-bool mix_flat_cached(const b200_ctx *ctx, const OperandView &v) {
+void plane_cache_drop_call_only(b200_ctx *ctx) {
+  PlaneCache &pc = ctx->planes;
+  std::vector<void *> blocks;
+  for (std::size_t i = 0; i < pc.entries.size();) {
+    if (pc.entries[i].call_only) {
+      blocks.push_back(pc.entries[i].block);
+      pc.bytes -= pc.entries[i].block_bytes;
+      pc.entries[i] = pc.entries.back();
+      pc.entries.pop_back();
+    } else {
+      ++i;
+    }
+  }
+  for (void *b : blocks) ctx->pool.free(b);
+}
+
+namespace {
+
+// What identifies a set of planes besides its kind: the array, and its line length where lines are padded.
+struct PlaneKey {
+  uint64_t elems;
+  std::size_t bytes;
+  uint32_t line, pad;   // line: 0 = element for element; pad: elements of a padded line
+  uint64_t lines;
+};
+
+PlaneKey plane_key(const OperandView &v, PlaneKind kind) {
+  PlaneKey key;
+  const uint32_t inner = v.mn_major ? v.mn : v.k;
+  key.lines = static_cast<uint64_t>(v.nbatch > 1 ? v.nbatch : 1u) * (v.mn_major ? v.k : v.mn);
+  key.pad = (inner + 7u) & ~7u;
+  key.line = kind == kPlanesMix && flat_exact(v) ? 0u : inner;
+  key.elems = key.lines * inner;
+  key.bytes = key.elems * (kind == kPlanesHalf ? 2u : 4u);
+  return key;
+}
+
+bool plane_match(const PlaneCache::Entry &e, const OperandView &v, PlaneKind kind, const PlaneKey &key) {
+  return e.src == v.ptr && e.src_bytes == key.bytes && e.kind == kind && e.line == key.line;
+}
+
+bool plane_cache_on(const PlaneCache &pc, PlaneKind kind) { return pc.scope > 0 || (kind == kPlanesMix && pc.cap != 0); }
+
+}  // namespace
+
+bool flat_cached(const b200_ctx *ctx, const OperandView &v, PlaneKind kind) {
   const PlaneCache &pc = ctx->planes;
-  if (!pc.active()) return false;
-  const uint64_t n = static_cast<uint64_t>(v.nbatch > 1 ? v.nbatch : 1u) * v.mn * v.k;
+  if (!plane_cache_on(pc, kind)) return false;
+  const PlaneKey key = plane_key(v, kind);
   for (const PlaneCache::Entry &e : pc.entries)
-    if (e.src == v.ptr && e.src_bytes == n * sizeof(float)) return true;
+    if (plane_match(e, v, kind, key)) return true;
   return false;
 }
 
-int mix_flat_planes(b200_ctx *ctx, cudaStream_t stream, const OperandView &v, const void *planes_out[3],
-                    void **owned_block) {
+int flat_planes(b200_ctx *ctx, cudaStream_t stream, OperandView &v, PlaneKind kind, const void *planes_out[3],
+                void **owned_block) {
   PlaneCache &pc = ctx->planes;
-  const uint64_t n = static_cast<uint64_t>(v.nbatch > 1 ? v.nbatch : 1u) * v.mn * v.k;
+  const PlaneKey key = plane_key(v, kind);
+  const uint64_t n = key.line ? key.lines * key.pad : key.elems;
   const uint64_t hi_elems = (n + 63ull) & ~63ull, h8_elems = (n + 127ull) & ~127ull;
-  const std::size_t block_bytes = hi_elems * sizeof(float) + 2 * h8_elems * sizeof(__nv_bfloat16);
+  const std::size_t block_bytes = kind == kPlanesHalf ? h8_elems * 2u
+                                  : kind == kPlanesTf32 ? hi_elems * sizeof(float)
+                                                        : hi_elems * sizeof(float) + 2 * h8_elems * sizeof(__nv_bfloat16);
+  const void *src = v.ptr;
   auto planes_of = [&](void *block) {
     float *hi = static_cast<float *>(block);
     __nv_bfloat16 *h8 = reinterpret_cast<__nv_bfloat16 *>(hi + hi_elems);
     planes_out[0] = hi;
-    planes_out[1] = h8;
-    planes_out[2] = h8 + h8_elems;
+    planes_out[1] = kind == kPlanesMix ? h8 : nullptr;
+    planes_out[2] = kind == kPlanesMix ? h8 + h8_elems : nullptr;
+    v.ptr = hi;
+    if (key.line) {
+      v.ld = key.pad;
+      v.batch_stride = static_cast<uint64_t>(key.pad) * (v.mn_major ? v.k : v.mn);
+    }
   };
   *owned_block = nullptr;
-  if (pc.active()) {
+  const bool active = plane_cache_on(pc, kind);
+  if (active) {
     for (PlaneCache::Entry &e : pc.entries) {
-      if (e.src == v.ptr && e.src_bytes == n * sizeof(float)) {
+      if (plane_match(e, v, kind, key)) {
         e.stamp = ++pc.clock;
         ++pc.hits;
         planes_of(e.block);
@@ -695,19 +792,32 @@ int mix_flat_planes(b200_ctx *ctx, cudaStream_t stream, const OperandView &v, co
   const int rc = ctx->pool.alloc(block_bytes, &block, nullptr);
   if (rc != B200_OK) return rc;
   planes_of(block);
+  void *p0 = block, *p1 = const_cast<void *>(planes_out[1]), *p2 = const_cast<void *>(planes_out[2]);
   {
     ProfScope prof(ctx, kProfPack, stream);
-    const unsigned long long n4 = n / 4ull;
     const unsigned long long cap = static_cast<unsigned long long>(ctx->sm_count) * 16ull;
-    const unsigned long long need = (n4 + 1023ull) / 1024ull;
-    b200::launch(ctx, pack_mix_flat_kernel, dim3(static_cast<unsigned>(need < cap ? need : cap)), dim3(256), 0, stream, 1u, static_cast<const float4 *>(v.ptr), reinterpret_cast<float4 *>(const_cast<void *>(planes_out[0])),
-        reinterpret_cast<uint2 *>(const_cast<void *>(planes_out[1])),
-        reinterpret_cast<uint2 *>(const_cast<void *>(planes_out[2])), n4);
+    if (key.line == 0u) {
+      const unsigned long long n4 = n / 4ull, need = (n4 + 1023ull) / 1024ull;
+      b200::launch(ctx, pack_mix_flat_kernel, dim3(static_cast<unsigned>(need < cap ? need : cap)), dim3(256), 0, stream, 1u,
+                   static_cast<const float4 *>(src), static_cast<float4 *>(p0), static_cast<uint2 *>(p1), static_cast<uint2 *>(p2), n4);
+    } else {
+      // lanes of a warp per line: enough for its pairs, at most all
+      uint32_t shift = 0;
+      while (shift < 5u && (2u << shift) < key.pad) ++shift;
+      const unsigned long long need = ((key.lines << shift) + 255ull) / 256ull;
+      const dim3 grid(static_cast<unsigned>(need < cap ? need : cap));
+      if (kind == kPlanesHalf)
+        b200::launch(ctx, pad_lines_kernel<kPlanesHalf, __half>, grid, dim3(256), 0, stream, 1u, static_cast<const __half *>(src), p0, p1, p2, key.line, key.pad, static_cast<unsigned long long>(key.lines), shift);
+      else if (kind == kPlanesTf32)
+        b200::launch(ctx, pad_lines_kernel<kPlanesTf32, float>, grid, dim3(256), 0, stream, 1u, static_cast<const float *>(src), p0, p1, p2, key.line, key.pad, static_cast<unsigned long long>(key.lines), shift);
+      else
+        b200::launch(ctx, pad_lines_kernel<kPlanesMix, float>, grid, dim3(256), 0, stream, 1u, static_cast<const float *>(src), p0, p1, p2, key.line, key.pad, static_cast<unsigned long long>(key.lines), shift);
+    }
   }
   ++ctx->launches;
   // inside an entry point that shares planes (scope) without a caller-set cap, keep at most 4 GiB
   const std::size_t cap = pc.cap ? pc.cap : (std::size_t(4) << 30);
-  if (!pc.active() || block_bytes > cap) {
+  if (!active || block_bytes > cap) {
     *owned_block = block;
     return B200_OK;
   }
@@ -721,7 +831,7 @@ int mix_flat_planes(b200_ctx *ctx, cudaStream_t stream, const OperandView &v, co
     pc.entries.pop_back();
     ctx->pool.free(old);
   }
-  pc.entries.push_back({v.ptr, static_cast<std::size_t>(n * sizeof(float)), block, block_bytes, ++pc.clock});
+  pc.entries.push_back({src, key.bytes, block, block_bytes, ++pc.clock, kind, key.line, kind != kPlanesMix});
   pc.bytes += block_bytes;
   return B200_OK;
 }

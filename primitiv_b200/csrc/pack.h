@@ -57,18 +57,27 @@ MixPlanes mix_planes(const OperandView &v);
 void pack_mix(b200_ctx *ctx, cudaStream_t stream, OperandView &v, float *dst, const MixPlanes &lay,
               const void *planes_out[3], bool hi_only = false);
 
-// Flat form of the same three planes: element e of the caller's array <-> element e of each plane,
-// so the planes keep the operand's major-ness and serve any later use of the same array.  Possible
-// when the operand is dense and every stride is a multiple of 8 elements (TMA needs 16-byte rows in
-// the bf16 planes too).
-bool mix_flat_ok(const OperandView &v);
-// Whether the context's plane cache already holds the flat planes of this operand.
-bool mix_flat_cached(const b200_ctx *ctx, const OperandView &v);
-// Finds the operand's flat planes in the context's plane cache, or packs them (one elementwise
-// pass) and offers them to the cache.  planes_out = {hi, hi8, lo8}.  *owned_block is the block the
-// caller has to return to the pool after its launch, or null when the cache keeps it.
-int mix_flat_planes(b200_ctx *ctx, cudaStream_t stream, const OperandView &v, const void *planes_out[3],
-                    void **owned_block);
+// ---- planes in the operand's own layout ----
+// Line by line copies of a dense operand that keep its major-ness and serve any later use of the same
+// array.  TMA needs lines of a multiple of 16 bytes (8 elements, with bf16 planes): where the operand's
+// lines are, and it is aligned, element e of the array is element e of each plane and the pass is purely
+// elementwise; otherwise lines are padded to the next multiple of 8 elements.
+enum PlaneKind : int {
+  kPlanesMix = 0,    // fp32 mode: {hi, hi8, lo8} as above
+  kPlanesTf32 = 1,   // single-pass TF32: one float plane, rounded
+  kPlanesHalf = 2,   // halves as they are, padded only
+};
+// Whether the operand is dense: lines back to back, matrices back to back.
+bool flat_ok(const OperandView &v);
+// Whether its planes would be element for element (no padding).
+bool flat_exact(const OperandView &v);
+// Whether the context's plane cache already holds them.
+bool flat_cached(const b200_ctx *ctx, const OperandView &v, PlaneKind kind);
+// Finds the planes in the context's plane cache, or packs them and offers them to the cache.  v is rewritten
+// to describe them (ptr, ld, batch_stride); planes_out = {hi, hi8, lo8} or {plane, null, null}.  *owned_block is
+// the block the caller has to return to the pool after its launch, or null when the cache keeps it.
+int flat_planes(b200_ctx *ctx, cudaStream_t stream, OperandView &v, PlaneKind kind, const void *planes_out[3],
+                void **owned_block);
 
 // ---- half planes of the 3xFP16 mode: [row maxima][h0 plane][h1 plane], rows of kpad halves ----
 struct F16Planes {
