@@ -209,7 +209,7 @@ B200_API int b200_matmul_fw_bw_host(b200_ctx *ctx, int mode,
  * loop of Sgemm calls, matmul.cu:113-123).
  * force_path: 0 = choose; 1 = CUDA-core kernel; 2 = tensor-core kernel (error if ineligible);
  * 3 = the CUDA-core kernels for one tiny extent (m <= 16 or k <= 16) against large ones (error if
- * the shape and layout are not one of theirs). */
+ * the shape and layout are not one of theirs); 4 = the mma.sync kernel. */
 B200_API int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b,
                        const void *A, const void *B, void *C,
                        uint32_t m, uint32_t n, uint32_t k,
@@ -321,7 +321,7 @@ B200_API int b200_set_correction_policy(b200_ctx *ctx, int policy);
  * bracketed by a pair of CUDA events on its stream.  b200_profile_read synchronises the
  * device, sums elapsed milliseconds and launch counts per kernel kind since the last
  * read, and clears the records:
- *   [0] tensor-core GEMM   [1] TF32 packing pre-pass   [2] CUDA-core GEMM   [3] elementwise */
+ *   [0] tcgen05 GEMM   [1] packing pre-pass   [2] the other GEMM kernels (mma.sync, CUDA cores)   [3] elementwise */
 B200_API int b200_profile_enable(b200_ctx *ctx, int on);
 B200_API int b200_profile_read(b200_ctx *ctx, double ms[4], uint64_t launches[4]);
 

@@ -308,24 +308,22 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   if (force_path == 2) return eligible ? b200::gemm_tc(ctx, g, s) : B200_ERR_INVALID_ARG;
   if (force_path == 1) return b200::gemm_simt(ctx, g, s);
   if (force_path == 3) return b200::gemm_skinny_eligible(g) ? b200::gemm_skinny(ctx, g, s) : B200_ERR_INVALID_ARG;
+  if (force_path == 4) return b200::gemm_mma(ctx, g, s);
   if (ctx->path_policy == 2 && eligible) return b200::gemm_tc(ctx, g, s);
   if (ctx->path_policy == 1) return b200::gemm_simt(ctx, g, s);
-  // A 128-row MMA tile on a problem this small is mostly padding; the CUDA-core
-  // kernel wins below roughly a tile's worth of work.
-  // One tiny extent against large ones is HBM-bound.  In the fp32-grade modes the tensor-core
-  // path would first pack the large operand into planes (three more passes over it): there the
-  // CUDA-core kernels that stream it once win (255-335 us against 675 us for the three products of
-  // a 10 x 1024 layer over 65536 items) and are exact fp32.  The single-pass modes need no
-  // packing and stay on the tensor-core path where TMA's alignment rules admit the operands; where
-  // they do not (ten rows of halves are 20 bytes) the alternative is the general CUDA-core kernel,
-  // which takes 5.8 ms for the reduce shape against 0.12 ms here.
-  if ((mode == B200_MODE_FP32_3XTF32 || mode == B200_MODE_FP32_3XFP16 || !eligible) && b200::gemm_skinny_eligible(g))
-    return b200::gemm_skinny(ctx, g, s);
-  const double macs = static_cast<double>(m) * n * k * groups * red;
-  // (a few rows against a long contraction are still worth it: the tensor-core path splits k
-  // over all SMs and streams the big operand once, the CUDA-core kernel would run on a few CTAs)
-  if (eligible && n >= 16 && macs >= 2097152.0 && (m >= 32 || macs >= 67108864.0)) return b200::gemm_tc(ctx, g, s);
-  return b200::gemm_simt(ctx, g, s);
+  // One tiny extent against large ones is HBM-bound.  Where the tensor-core path would first have to pack
+  // the large operand (always in the fp32-grade modes: three more passes over it), the CUDA-core
+  // kernels that stream it once win (255-335 us against 675 us for the three products of a 10 x 1024
+  // layer over 65536 items) and are exact fp32.
+  if (b200::gemm_skinny_eligible(g) && !b200::gemm_tc_reads_in_place(ctx, g)) return b200::gemm_skinny(ctx, g, s);
+  // Below two million multiply-adds a 128-row tcgen05 tile is mostly padding.  A contraction of a few terms
+  // would not even fill a k-step of mma.sync (800 x 200 x 10: 3.4 us on the CUDA cores, 4.1 us there).
+  if (static_cast<double>(m) * n * k * groups * red < 2097152.0)
+    return static_cast<uint64_t>(k) * red <= 16u ? b200::gemm_simt(ctx, g, s) : b200::gemm_mma(ctx, g, s);
+  // Large products belong to tcgen05, small, thin and ragged ones to mma.sync (gemm_mma.cuh): whichever is
+  // estimated to take less.
+  if (b200::gemm_mma_estimate(ctx, g) < b200::gemm_tc_estimate(ctx, g)) return b200::gemm_mma(ctx, g, s);
+  return b200::gemm_tc(ctx, g, s);
 }
 
 int b200_gemm_3xtf32_noalloc(b200_ctx *ctx, int trans_a, int trans_b, const void *A, const void *B,

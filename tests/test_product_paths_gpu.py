@@ -1,0 +1,78 @@
+"""b200_gemm on one path at a time, at the sizes where tiles, splits and loads have their edges, in every
+operand layout, against an fp64 product of the values the device stores."""
+import pytest
+import torch
+
+from gpu_util import MODES, TOL
+
+pytestmark = pytest.mark.gpu
+
+# (m, n, k, groups, red): extents at, below and above the tiles (8, 16, 32, 64, 128 columns, 64 and 128 rows,
+# k-tiles of 32 floats / 64 halves), the exchanged form (m <= 32 < n), splits over a cluster and over scratch
+SIZES = [
+    (1, 1, 17, 1, 1), (128, 8, 512, 1, 1), (129, 9, 513, 1, 1), (130, 16, 1000, 2, 1), (10, 300, 77, 1, 1), (33, 31, 4096, 1, 1),
+    (256, 256, 256, 1, 1), (64, 64, 64, 3, 1), (65, 63, 33, 3, 1), (200, 136, 264, 1, 3), (515, 387, 201, 2, 1), (384, 320, 2048, 1, 1),
+]
+
+
+def product(a, b, ta, tb, m, n, k):
+    """Column-major opA(a) . opB(b) of flat arrays, as a flat array."""
+    a = a.view(m, k) if ta else a.view(k, m).T
+    b = b.view(k, n).T if tb else b.view(n, k)      # n x k
+    return (b @ a.T).reshape(-1)                     # n rows of m: column-major m x n
+
+
+@pytest.mark.parametrize("path", [2, 4], ids=["tcgen05", "mma_sync"])
+@pytest.mark.parametrize("mode", list(MODES))
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+def test_paths_at_their_edges(ctx, path, mode, layout):
+    ta, tb = (int(c == "t") for c in layout)
+    kind = torch.float16 if mode == "fp16" else torch.float32
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(7)
+    for m, n, k, groups, red in SIZES:
+        for offset in (0, 1):                        # 1: nothing is aligned
+            count = groups * red
+            a, b = (torch.randn(count * s + 1, device="cuda", generator=gen).to(kind)[offset:offset + count * s] for s in (m * k, k * n))
+            c = torch.randn(groups * m * n + 9, device="cuda", generator=gen).to(kind)[offset:]
+            before = c.clone()
+            accumulate = (m + n) % 2 == 0
+            ctx.gemm(MODES[mode], ta, tb, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, groups, red,
+                     m * k * red if groups > 1 else 0, m * k if red > 1 else 0, k * n * red if groups > 1 else 0,
+                     k * n if red > 1 else 0, m * n, accumulate, path)
+            assert ctx.status_poll() == 0
+            a, b, old = a.double().view(count, -1), b.double().view(count, -1), before.double()
+            want = torch.cat([sum(product(a[g * red + r], b[g * red + r], ta, tb, m, n, k) for r in range(red)) for g in range(groups)])
+            size = want.norm()                       # errors scale with the product, whatever it is added to
+            got = c[:groups * m * n].double() - (old[:groups * m * n] if accumulate else 0)
+            # half storage: the sum is rounded once, 2^-11 of its own size
+            slack = 2.0 ** -11 * (want + old[:groups * m * n]).norm() if mode == "fp16" and accumulate else 0.0
+            if m * n > 1:                            # (a single value may cancel to nothing)
+                assert (got - want).norm() <= TOL[mode] * size + slack, (m, n, k, groups, red, offset)
+            assert torch.equal(c[groups * m * n:], before[groups * m * n:]), "wrote past the result"
+
+
+@pytest.mark.parametrize("mode", ["fp16", "tf32", "3xtf32"])
+def test_padded_lines_are_shared_inside_one_backward_call(ctx, mode):
+    """Operands whose lines TMA cannot address: gy's padded copy serves both gradients of one call (one
+    hit), and nothing of it outlives the call."""
+    di, dj, dk, n = 515, 389, 131, 6
+    kind = torch.float16 if mode == "fp16" else torch.float32
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(3)
+    a, b, gy = (torch.randn(n * s, device="cuda", generator=gen).to(kind) for s in (di * dj, dj * dk, di * dk))
+    ga, gb = torch.empty_like(a), torch.empty_like(b)
+    ctx.set_path_policy(2)
+    try:
+        s0 = ctx.operand_cache_stats()
+        ctx.matmul_bw_ex(MODES[mode], a.data_ptr(), b.data_ptr(), gy.data_ptr(), ga.data_ptr(), gb.data_ptr(), di, dj, dk, n, n,
+                         False, False)
+        s1 = ctx.operand_cache_stats()
+    finally:
+        ctx.set_path_policy(0)
+    assert s1["hits"] - s0["hits"] == 1 and s1["entries"] == 0, (s0, s1)
+    a64, b64, gy64 = a.double().view(n, dj, di), b.double().view(n, dk, dj), gy.double().view(n, dk, di)
+    want_a = torch.einsum("nki,nkj->nji", gy64, b64)
+    want_b = torch.einsum("nji,nki->nkj", a64, gy64)
+    for got, want in ((ga, want_a), (gb, want_b)):
+        assert (got.double().view_as(want) - want).norm() <= TOL[mode] * want.norm()
