@@ -309,6 +309,7 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   if (force_path == 1) return b200::gemm_simt(ctx, g, s);
   if (force_path == 3) return b200::gemm_skinny_eligible(g) ? b200::gemm_skinny(ctx, g, s) : B200_ERR_INVALID_ARG;
   if (force_path == 4) return b200::gemm_mma(ctx, g, s);
+  if (force_path == 5) return b200::gemm_direct(ctx, g, s);
   if (ctx->path_policy == 2 && eligible) return b200::gemm_tc(ctx, g, s);
   if (ctx->path_policy == 1) return b200::gemm_simt(ctx, g, s);
   // One tiny extent against large ones is HBM-bound.  Where the tensor-core path would first have to pack
@@ -320,10 +321,11 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   // would not even fill a k-step of mma.sync (800 x 200 x 10: 3.4 us on the CUDA cores, 4.1 us there).
   if (static_cast<double>(m) * n * k * groups * red < 2097152.0)
     return static_cast<uint64_t>(k) * red <= 16u ? b200::gemm_simt(ctx, g, s) : b200::gemm_mma(ctx, g, s);
-  // Large products belong to tcgen05, small, thin and ragged ones to mma.sync (gemm_mma.cuh): whichever is
-  // estimated to take less.
-  if (b200::gemm_mma_estimate(ctx, g) < b200::gemm_tc_estimate(ctx, g)) return b200::gemm_mma(ctx, g, s);
-  return b200::gemm_tc(ctx, g, s);
+  // Large products belong to tcgen05 fed by TMA, small fp32 ones to tcgen05 fed by the kernel's own loads, thin and
+  // ragged ones to mma.sync: whichever is estimated to take least.
+  const double tc = b200::gemm_tc_estimate(ctx, g), mma = b200::gemm_mma_estimate(ctx, g), direct = b200::gemm_direct_estimate(ctx, g);
+  if (direct < tc && direct < mma) return b200::gemm_direct(ctx, g, s);
+  return mma < tc ? b200::gemm_mma(ctx, g, s) : b200::gemm_tc(ctx, g, s);
 }
 
 int b200_gemm_3xtf32_noalloc(b200_ctx *ctx, int trans_a, int trans_b, const void *A, const void *B,

@@ -234,6 +234,8 @@ bool gemm_skinny_eligible(const GemmArgs &g);
 int gemm_skinny(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // mma.sync path: any shape, any alignment, operands read where they lie (gemm_mma.cuh).
 int gemm_mma(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
+// fp32 modes, tcgen05 fed by the kernel's own loads: any shape, any alignment (gemm_direct.cu).
+int gemm_direct(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // tcgen05 path.  tc_eligible() says whether the operands meet TMA's alignment rules.
 bool gemm_tc_eligible(const b200_ctx *ctx, const GemmArgs &g);
 int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
@@ -243,6 +245,7 @@ bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g);
 // between them.  1e30: not eligible.
 double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g);
+double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g);
 // Checks (and re-arms) the guard bands of every pool block; see b200_pool_check_guards.
 int pool_check_guards(b200_ctx *ctx, cudaStream_t stream, std::uint64_t *damaged, void **first, int *side);
 // Streams L2-resident data into every SM's shared memory and reports the rate; see b200_measure_l2_ingest.
