@@ -93,6 +93,12 @@ int b200_ctx_create(int device_id, b200_ctx **out) {
     delete ctx;
     return B200_ERR_DRIVER;
   }
+  const int rc = b200::gemm_direct_init(ctx);
+  if (rc != B200_OK) {
+    cudaFreeHost(ctx->h_status);
+    delete ctx;
+    return rc;
+  }
   *out = ctx;
   return B200_OK;
 }
@@ -323,7 +329,10 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
     return static_cast<uint64_t>(k) * red <= 16u ? b200::gemm_simt(ctx, g, s) : b200::gemm_mma(ctx, g, s);
   // Large products belong to tcgen05 fed by TMA, small fp32 ones to tcgen05 fed by the kernel's own loads, thin and
   // ragged ones to mma.sync: whichever is estimated to take least.
-  const double tc = b200::gemm_tc_estimate(ctx, g), mma = b200::gemm_mma_estimate(ctx, g), direct = b200::gemm_direct_estimate(ctx, g);
+  const double tc = b200::gemm_tc_estimate(ctx, g), direct = b200::gemm_direct_estimate(ctx, g);
+  double mma = b200::gemm_mma_estimate(ctx, g);
+  // (near ties go to the kernels that share one order of summation: the estimates are no better than that)
+  if (b200::gemm_fixed_slices(ctx, g)) mma *= 1.1;
   if (direct < tc && direct < mma) return b200::gemm_direct(ctx, g, s);
   return mma < tc ? b200::gemm_mma(ctx, g, s) : b200::gemm_tc(ctx, g, s);
 }

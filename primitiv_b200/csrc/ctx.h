@@ -136,6 +136,7 @@ struct b200_ctx {
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
   std::size_t smem_optin = 0;
+  int cluster_room[9] = {};      // clusters of 1 to 8 CTAs that run at a time with an SM to each CTA
   b200::Pool pool;
   // Status word of the bounded device-side waits.  It lives in pinned host memory that the
   // GPU writes through a mapped alias (d_status): a kernel whose wait ran out stores its code
@@ -221,7 +222,7 @@ struct GemmArgs {
 };
 
 // Tiny and thin products are bound by latency or by the large operand's bytes: even in TF32 mode they are
-// given fp32-grade arithmetic, which costs next to nothing there.
+// given fp32 arithmetic, or as good a split (gemm_mma.cuh), which costs next to nothing there.
 inline bool tiny_or_thin(const GemmArgs &g) {
   const double macs = static_cast<double>(g.m) * g.n * g.k * g.groups * g.red;
   return macs < 2097152.0 || g.n < 16u || (g.m < 32u && macs < 67108864.0);
@@ -236,6 +237,7 @@ int gemm_skinny(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 int gemm_mma(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // fp32 modes, tcgen05 fed by the kernel's own loads: any shape, any alignment (gemm_direct.cu).
 int gemm_direct(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
+int gemm_direct_init(b200_ctx *ctx);   // fills cluster_room
 // tcgen05 path.  tc_eligible() says whether the operands meet TMA's alignment rules.
 bool gemm_tc_eligible(const b200_ctx *ctx, const GemmArgs &g);
 int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
@@ -246,6 +248,8 @@ bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g);
+// The number of slices that every tcgen05 kernel cuts this contraction into; 0: each kernel as it likes.
+uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g);
 // Checks (and re-arms) the guard bands of every pool block; see b200_pool_check_guards.
 int pool_check_guards(b200_ctx *ctx, cudaStream_t stream, std::uint64_t *damaged, void **first, int *side);
 // Streams L2-resident data into every SM's shared memory and reports the rate; see b200_measure_l2_ingest.

@@ -8,12 +8,18 @@
 // step).  Here eight warps fetch operands with ordinary loads, of any alignment, split each element
 // once, and store the planes where the tensor core reads them; the same warps write the result.
 //
-// A step of 128 x 64 x 32 takes 0.62 us: 48 KB of planes are stored and read again by the tensor core and 24 KB of
+// A step of 128 x 64 x 32 takes 0.68 us: 48 KB of planes are stored and read again by the tensor core and 24 KB of
 // operands come in, and at 128 bytes per clock that is what shared memory moves.  TMA-fed planes need half of
-// that, so large products stay with gemm_tc.cu.  Measured in a chain of small kernels, planes and reduction
-// included: 800 x 200 x 784 14.1 -> 9.4 us, 800 x 784 x 200 14.5 -> 6.8, 512^3 14.7 -> 6.9, 256 x 1024 x 256 12.0 -> 5.7
-// (gemm_mma.cuh: 15.4, 15.1, 10.5, 7.3).  (128-column tiles, and the same kernel for halves and TF32, were built
-// too and were never the fastest.)
+// that, so large products stay with gemm_tc.cu.  Measured back to back, planes and reduction included, against
+// gemm_tc.cu: 800 x 200 x 784 14.9 -> 11.2 us, 800 x 784 x 200 12.9 -> 8.5, 512^3 16.0 -> 8.4, 256 x 1024 x 256
+// 12.3 -> 8.2 (gemm_mma.cuh: 17.5, 18.3, 13.0, 9.0).  Slices follow gemm_fixed_slices; tiles of 96 columns let
+// the 5 slices of 800 x 200 run at once (21 clusters, 26 fit; 64 columns make 28), tiles of 32 give unsplit
+// products more CTAs.  (128-column tiles, and the same kernel for halves and TF32, were built too and were
+// never the fastest.)
+//
+// The corrections of the default fp32 mode are bf16, with gemm_tc.cu's bits (off by 0.7 to 1.4e-6).  The 3xFP16 mode
+// promises 22 bits: its corrections are TF32 and have an accumulator of their own, and chunks are two k-blocks:
+// 2e-7 whatever the length, where its planes lose 2.8e-7 at 86 terms and 1.5e-6 at 784.
 //
 // Thread roles (288 threads): warps 0-7 feed stages and later drain the accumulator, warp 8 issues the MMAs.
 // A stage is one k-block of 32: [A hi | A hi8 | A lo8 | B hi | B hi8 | B lo8], hi in TF32, the correction operands
@@ -22,7 +28,7 @@
 //
 // The contraction of a tile may be cut over the CTAs of a cluster; their tiles meet through distributed
 // shared memory and are added in rank order: the same bits every run.  The accumulator is added to registers
-// every 8 k-blocks (the tensor core truncates when it accumulates, see gemm_tc.cu), one chunk behind the
+// every few k-blocks (the tensor core truncates when it accumulates, see gemm_tc.cu), one chunk behind the
 // feeding so that it never waits.
 #include <cuda_bf16.h>
 
@@ -44,6 +50,7 @@ struct DirectParams {
   uint32_t splits;                  // CTAs of a cluster that share a tile's contraction
   uint32_t kb, red;                 // k-blocks of one matrix pair, and pairs
   uint32_t kb_all, kb_per;          // k-blocks in all (red * kb), and of one split
+  uint32_t chunk;                   // k-blocks that the tensor core accumulates before their sum goes to registers: even
   unsigned long long lda, ldb;      // elements from one line to the next
   unsigned long long a_gs, a_rs, b_gs, b_rs, c_gs;
   uint32_t wide_a, wide_b;          // every line starts on 16 bytes
@@ -51,16 +58,17 @@ struct DirectParams {
   int *status;
 };
 
-constexpr uint32_t kDirectM = 128, kDirectN = 64, kDirectK = 32;
+constexpr uint32_t kDirectM = 128, kDirectK = 32;   // (a tile has 32, 64 or 96 columns)
 constexpr uint32_t kFeedThreads = 256, kFeedWarps = 8;
-constexpr uint32_t kDirectChunk = 8;   // k-blocks per accumulation chunk of the fp32 mode
 
 // One operand's tile: geometry of the shared-memory planes and of the feeding threads' share.
-template <bool kKMajor, uint32_t ROWS>
+// kFull: the second plane is x - hi in TF32 instead of two in bf16.
+template <bool kKMajor, uint32_t ROWS, bool kFull>
 struct Feed {
   static constexpr uint32_t kUnits = ROWS * 8u / kFeedThreads;          // units of four floats per thread and k-block
-  static constexpr uint32_t kPlane = ROWS * 128u, kPlane8 = ROWS * 64u;  // bytes of the main plane, of a bf16 plane
-  static constexpr uint32_t kBytes = 2u * kPlane;
+  static constexpr uint32_t kPlane = ROWS * 128u;                       // bytes of the main plane, of a bf16 plane
+  static constexpr uint32_t kPlane8 = (!kKMajor && ROWS < 64u ? 64u : ROWS) * 64u;   // (a line of 32 fills half of the swizzle's 128 bytes)
+  static constexpr uint32_t kBytes = kPlane + 2u * kPlane8;
   static constexpr uint32_t kLineUnits = kKMajor ? 8u : ROWS / 4u;    // units per line in memory
   static constexpr uint32_t kLineStep = kFeedThreads / kLineUnits;      // lines from one of a thread's units to the next
 
@@ -125,6 +133,11 @@ struct Feed {
     for (uint32_t i = 0; i < kUnits; ++i) {
       const float4 x = raw[i], hi = make_float4(round(x.x), round(x.y), round(x.z), round(x.w));
       asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(base + to + i * kToStep), "f"(hi.x), "f"(hi.y), "f"(hi.z), "f"(hi.w) : "memory");
+      if constexpr (kFull) {
+        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(base + kPlane + to + i * kToStep), "f"(round(x.x - hi.x)), "f"(round(x.y - hi.y)),
+                     "f"(round(x.z - hi.z)), "f"(round(x.w - hi.w)) : "memory");
+        continue;
+      }
       sts64(base + kPlane + to8 + i * kTo8Step, bf16x2(x.x, x.y), bf16x2(x.z, x.w));
       sts64(base + kPlane + kPlane8 + to8 + i * kTo8Step, bf16x2(x.x - hi.x, x.y - hi.y), bf16x2(x.z - hi.z, x.w - hi.w));
     }
@@ -154,17 +167,22 @@ __device__ __forceinline__ MixDesc plane_desc(bool tf32) {
   return d;
 }
 
-constexpr uint32_t kDirectStage = (kDirectM + kDirectN) * 256u;   // 48 KB
+template <bool KA, bool KB, uint32_t N>
+constexpr uint32_t kDirectStage = Feed<KA, kDirectM, false>::kBytes + Feed<KB, N, false>::kBytes;   // 40 to 56 KB
 constexpr uint32_t kDirectStages = 4;
 constexpr uint32_t kDirectPitch = kDirectM + 4u;                  // floats per column of the result tile
-constexpr uint32_t kDirectSmem = kDirectStages * kDirectStage + 1024u;   // (the result tile fits in it)
+template <bool KA, bool KB, uint32_t N>
+constexpr uint32_t kDirectSmem = kDirectStages * kDirectStage<KA, KB, N> + 1024u;   // (the result tile fits in it)
 
-template <bool KA, bool KB>
+template <bool KA, bool KB, uint32_t kDirectN, bool kFull>
 __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const __grid_constant__ DirectParams p) {
-  using FA = Feed<KA, kDirectM>;
-  using FB = Feed<KB, kDirectN>;
-  constexpr uint32_t kStages = kDirectStages, kHalfCols = kDirectN / 2u, kCols = 2u * kDirectN;   // two accumulators
-  static_assert(kHalfCols == 32u, "one tensor-memory load per chunk and warp");
+  using FA = Feed<KA, kDirectM, kFull>;
+  using FB = Feed<KB, kDirectN, kFull>;
+  constexpr uint32_t kStages = kDirectStages, kHalfCols = kDirectN / 2u;
+  constexpr uint32_t kSums = kFull ? 3u : 2u;   // accumulators: two in turn, one of the small terms
+  constexpr uint32_t kCols = kSums * kDirectN <= 64u ? 64u : kSums * kDirectN <= 128u ? 128u : kSums * kDirectN <= 256u ? 256u : 512u;
+  constexpr uint32_t kStageBytes = kDirectStage<KA, KB, kDirectN>;
+  static_assert(kDirectN == 32u || kDirectN == 64u || (kDirectN == 96u && KB), "what the feeding threads divide evenly");
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kStages];
   __shared__ __align__(8) uint64_t empty_bar[kStages];
@@ -205,7 +223,7 @@ __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const
   const uint32_t m0 = (rem % p.tiles_m) * kDirectM, n0 = (rem / p.tiles_m) * kDirectN;
   const uint32_t kb0 = rank * p.kb_per;
   const uint32_t count = kb0 + p.kb_per < p.kb_all ? p.kb_per : p.kb_all - kb0;   // > 0: the host makes no empty split
-  const uint32_t chunks = (count + kDirectChunk - 1u) / kDirectChunk;
+  const uint32_t chunks = (count + p.chunk - 1u) / p.chunk;
 
   const uint32_t quarter = warp & 3u, half = warp >> 2;            // tensor-memory lanes and columns of a feeding warp
   const uint32_t taddr = tmem + ((quarter * 32u) << 16) + half * kHalfCols;
@@ -235,7 +253,7 @@ __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const
     auto put = [&](const float4 (&ra)[FA::kUnits], const float4 (&rb)[FB::kUnits]) {
       ok = ok && mbar_wait(smem_u32(&empty_bar[stage]), phase ^ 1u, abort_flag);
       if (ok) {
-        const uint32_t at = base + stage * kDirectStage;
+        const uint32_t at = base + stage * kStageBytes;
         fa.store(ra, at);
         fb.store(rb, at + FA::kBytes);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor core reads through the async proxy
@@ -247,16 +265,28 @@ __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const
         phase ^= 1u;
       }
     };
+    auto add = [&](uint32_t cols, bool first) {
+      if constexpr (kHalfCols >= 32u) {
+        uint32_t v[32];
+        tmem_ld32(taddr + cols, v);
+#pragma unroll
+        for (uint32_t i = 0; i < 32u; ++i) sum[i] = first ? __uint_as_float(v[i]) : sum[i] + __uint_as_float(v[i]);
+      }
+      if constexpr (kHalfCols % 32u != 0u) {
+        constexpr uint32_t at = kHalfCols - 16u;
+        uint32_t v[16];
+        tmem_ld16(taddr + cols + at, v);
+#pragma unroll
+        for (uint32_t i = 0; i < 16u; ++i) sum[at + i] = first ? __uint_as_float(v[i]) : sum[at + i] + __uint_as_float(v[i]);
+      }
+    };
     // adds chunk c of the accumulator to the registers
     auto drain = [&](uint32_t c) {
       const uint32_t buf = c & 1u;
       ok = __all_sync(0xffffffffu, ok && mbar_wait(smem_u32(&acc_full_bar[buf]), (c >> 1) & 1u, abort_flag));
       if (!ok) return;
       tc_fence_after();
-      uint32_t v[32];
-      tmem_ld32(taddr + buf * kDirectN, v);
-#pragma unroll
-      for (uint32_t i = 0; i < 32u; ++i) sum[i] = c == 0u ? __uint_as_float(v[i]) : sum[i] + __uint_as_float(v[i]);
+      add(buf * kDirectN, c == 0u);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&acc_empty_bar[buf]));
@@ -275,10 +305,13 @@ __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const
         if (i + 3u < count) fetch(a1, b1);
       }
       // (chunks are an even number of k-blocks) one whole chunk is ahead of the one drained here
-      if (i + 2u == (drained + 2u) * kDirectChunk) drain(drained++);
+      if (i + 2u == (drained + 2u) * p.chunk) drain(drained++);
     }
 #pragma unroll 1
     while (drained < chunks) drain(drained++);
+    if constexpr (kFull) {
+      if (ok) add(2u * kDirectN, false);
+    }
   } else {
     const MixDesc da = plane_desc<KA>(true), db = plane_desc<KB>(true), da8 = plane_desc<KA>(false), db8 = plane_desc<KB>(false);
     constexpr uint32_t kShape = (1u << 4) | ((KA ? 0u : 1u) << 15) | ((KB ? 0u : 1u) << 16) | ((kDirectN >> 3) << 17) | ((kDirectM >> 4) << 24);
@@ -292,7 +325,7 @@ __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const
       if (!ok) break;
       tc_fence_after();
       const uint32_t d = tmem + buf * kDirectN;
-      const uint32_t n = left > kDirectChunk ? kDirectChunk : left;
+      const uint32_t n = left > p.chunk ? p.chunk : left;
       left -= n;
 #pragma unroll 1
       for (uint32_t i = 0; i < n; ++i) {
@@ -301,8 +334,14 @@ __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const
           break;
         }
         tc_fence_after();
-        const uint32_t sa = base + stage * kDirectStage, sb = sa + FA::kBytes;
-        mma_stage_mix<1>(d, sa, sb, FA::kPlane, FB::kPlane, FA::kPlane8, FB::kPlane8, da, da8, db, db8, kIdesc, kIdesc8, i == 0u);
+        const uint32_t sa = base + stage * kStageBytes, sb = sa + FA::kBytes;
+        if constexpr (kFull) {
+          const uint32_t small = tmem + 2u * kDirectN;
+          mma_stage<1, false, 1>(small, sa + FA::kPlane, sb, 0u, 0u, da.hi, db.hi, da.lo_fixed, db.lo_fixed, da.kstep, db.kstep, kIdesc, c + i == 0u);
+          mma_stage<1, false, 1>(small, sa, sb + FB::kPlane, 0u, 0u, da.hi, db.hi, da.lo_fixed, db.lo_fixed, da.kstep, db.kstep, kIdesc, false);
+          mma_stage<1, false, 1>(d, sa, sb, 0u, 0u, da.hi, db.hi, da.lo_fixed, db.lo_fixed, da.kstep, db.kstep, kIdesc, i == 0u);
+        } else
+          mma_stage_mix<1>(d, sa, sb, FA::kPlane, FB::kPlane, FA::kPlane8, FB::kPlane8, da, da8, db, db8, kIdesc, kIdesc8, i == 0u);
         mma_commit(smem_u32(&empty_bar[stage]));
         if (++stage == kStages) {
           stage = 0;
@@ -395,37 +434,59 @@ __global__ void __launch_bounds__(kFeedThreads + 32, 1) gemm_direct_kernel(const
   }
 }
 
-template <bool KA, bool KB>
+template <bool KA, bool KB, uint32_t N, bool kFull>
 int direct_launch(b200_ctx *ctx, const DirectParams &p, cudaStream_t stream) {
-  auto kernel = gemm_direct_kernel<KA, KB>;
+  auto kernel = gemm_direct_kernel<KA, KB, N, kFull>;
+  constexpr uint32_t kSmem = kDirectSmem<KA, KB, N>;
   static std::atomic<unsigned long long> done{0};   // opted in to large shared memory, one bit per device
   const unsigned long long bit = 1ull << (ctx->device & 63);
   if (!(done.load(std::memory_order_relaxed) & bit)) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDirectSmem));
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem));
     if (e != cudaSuccess) return static_cast<int>(e);
     done.fetch_or(bit, std::memory_order_relaxed);
   }
   const unsigned grid = p.tiles_m * p.tiles_n * p.groups * p.splits;
-  b200::launch(ctx, kernel, dim3(grid), dim3(kFeedThreads + 32u), kDirectSmem, stream, p.splits, p);
+  b200::launch(ctx, kernel, dim3(grid), dim3(kFeedThreads + 32u), kSmem, stream, p.splits, p);
   return static_cast<int>(cudaGetLastError());
 }
 
+template <bool KA, bool KB, bool kFull>
+int direct_launch(b200_ctx *ctx, const DirectParams &p, uint32_t cols, cudaStream_t stream) {
+  if constexpr (KB) {
+    if (cols == 96u) return direct_launch<KA, true, 96u, kFull>(ctx, p, stream);
+  }
+  return cols == 32u ? direct_launch<KA, KB, 32u, kFull>(ctx, p, stream) : direct_launch<KA, KB, 64u, kFull>(ctx, p, stream);
+}
+
+template <bool kFull>
+int direct_launch(b200_ctx *ctx, const DirectParams &p, bool ka, bool kb, uint32_t cols, cudaStream_t stream) {
+  if (ka) return kb ? direct_launch<true, true, kFull>(ctx, p, cols, stream) : direct_launch<true, false, kFull>(ctx, p, cols, stream);
+  return kb ? direct_launch<false, true, kFull>(ctx, p, cols, stream) : direct_launch<false, false, kFull>(ctx, p, cols, stream);
+}
+
 struct DirectChoice {
-  uint32_t splits;
+  uint32_t cols, splits;
   double us;
 };
 
-// One CTA fits on an SM; a k-block takes 0.66 us (0.9 us where loads are single floats), a tile 3.5 us besides with
-// its launch, adding up a split 1.7 us.  A cluster has to fit a GPC, so a split fills at most 7/8 of the GPU.
+// One CTA fits on an SM; a k-block takes 0.56, 0.68 or 1.0 us (more where loads are single floats), a tile 2 us
+// besides, 2.9 where others follow it, adding up a split 1.7 us: fitted to 60 products.  A cluster has to fit a
+// GPC: of 28 clusters of five only 26 run at a time (ctx->cluster_room).
 DirectChoice choose(const b200_ctx *ctx, const GemmArgs &g, bool wide) {
-  const double tiles = static_cast<double>((g.m + kDirectM - 1) / kDirectM) * ((g.n + kDirectN - 1) / kDirectN) * g.groups;
+  static const struct { uint32_t cols; double wide, narrow; } kTiles[] = {{64, 0.68, 0.8}, {96, 1.0, 1.1}, {32, 0.56, 0.7}};
   const uint64_t kb = static_cast<uint64_t>((g.k + kDirectK - 1) / kDirectK) * g.red;
-  DirectChoice best{1, 1e30};
-  for (uint32_t s = 1; s <= 8u && s <= kb; ++s) {
-    if (s > 1u && tiles * s > ctx->sm_count * 0.875) break;
-    const double waves = static_cast<double>(static_cast<uint64_t>((tiles * s + ctx->sm_count - 1) / ctx->sm_count));
-    const double us = 1.5 + waves * (static_cast<double>((kb + s - 1) / s) * (wide ? 0.66 : 0.9) + 2.0) + (s > 1u ? 1.7 : 0.0);
-    if (us < best.us) best = {s, us};
+  const uint32_t fixed = gemm_fixed_slices(ctx, g);
+  DirectChoice best{64, fixed ? fixed : 1u, 1e30};
+  for (const auto &t : kTiles) {
+    if (t.cols == 96u && g.trans_b) continue;   // (a line of 96 columns does not divide among the threads)
+    const double tiles = static_cast<double>((g.m + kDirectM - 1) / kDirectM) * ((g.n + t.cols - 1) / t.cols) * g.groups;
+    for (uint32_t s = 1; s <= 8u && s <= kb; ++s) {
+      const double room = ctx->cluster_room[s];
+      if (fixed ? s != fixed : (s > 1u && tiles > room)) continue;
+      const double waves = static_cast<double>(static_cast<uint64_t>((tiles + room - 1) / room));
+      const double us = 1.5 + waves * (static_cast<double>((kb + s - 1) / s) * (wide ? t.wide : t.narrow) + (waves > 1.0 ? 2.9 : 2.0) + (s > 1u ? 1.7 : 0.0));
+      if (us < best.us) best = {t.cols, s, us};
+    }
   }
   return best;
 }
@@ -441,7 +502,32 @@ bool wide_b(const GemmArgs &g) { return all_wide(g.B, g.trans_b ? g.n : g.k, g.b
 double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g) {
   if (g.mode != B200_MODE_FP32_3XTF32 && g.mode != B200_MODE_FP32_3XFP16) return 1e30;
   if (ctx->correction_policy == 1) return 1e30;   // the caller wants TF32 planes throughout
+  if (tiny_or_thin(g)) return 1e30;
+  // (half planes lose less than this kernel where the sum is that short: 1.2e-7 against 1.6e-7 at 48 terms)
+  if (g.mode == B200_MODE_FP32_3XFP16 && static_cast<uint64_t>(g.k) * g.red < 64u) return 1e30;
   return choose(ctx, g, wide_a(g) && wide_b(g)).us;
+}
+
+int gemm_direct_init(b200_ctx *ctx) {
+  auto kernel = gemm_direct_kernel<true, true, 64u, false>;
+  constexpr uint32_t kSmem = kDirectSmem<true, true, 64u>;
+  B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
+  ctx->cluster_room[1] = ctx->sm_count;
+  for (unsigned s = 2; s <= 8u; ++s) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = s;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(s);
+    cfg.blockDim = dim3(kFeedThreads + 32u);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    B200_CUDA_TRY(cudaOccupancyMaxActiveClusters(&ctx->cluster_room[s], kernel, &cfg));
+    if (ctx->cluster_room[s] < 1) ctx->cluster_room[s] = 1;
+  }
+  return B200_OK;
 }
 
 int gemm_direct(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream) {
@@ -466,18 +552,22 @@ int gemm_direct(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream) {
   if (all > 0x7fffffffull) return B200_ERR_TOO_LARGE;
   p.kb_all = static_cast<uint32_t>(all);
   p.tiles_m = (g.m + kDirectM - 1) / kDirectM;
-  p.tiles_n = (g.n + kDirectN - 1) / kDirectN;
-  uint32_t splits = choose(ctx, g, p.wide_a && p.wide_b).splits;
+  const DirectChoice c = choose(ctx, g, p.wide_a && p.wide_b);
+  uint32_t splits = c.splits, cols = c.cols;
 #ifdef PRIMITIV_B200_DEV_KNOBS
+  if (const char *e = std::getenv("PRIMITIV_B200_DIRECT_COLS")) cols = std::atoi(e) == 32 ? 32u : std::atoi(e) == 96 && !g.trans_b ? 96u : 64u;
   if (const char *e = std::getenv("PRIMITIV_B200_DIRECT_SPLITS")) splits = std::atoi(e);
 #endif
+  p.tiles_n = (g.n + cols - 1) / cols;
+  // (longer chunks truncate more: where the order is not fixed, shorter ones cost next to nothing)
+  p.chunk = g.mode == B200_MODE_FP32_3XFP16 ? 2u : gemm_fixed_slices(ctx, g) ? 8u : 4u;
   p.kb_per = (p.kb_all + splits - 1) / splits;
   p.splits = (p.kb_all + p.kb_per - 1) / p.kb_per;   // no empty splits
   if (static_cast<uint64_t>(p.tiles_m) * p.tiles_n * g.groups * p.splits > 0x7fffffffull) return B200_ERR_TOO_LARGE;
   ProfScope prof(ctx, kProfGemmTc, stream);
   ++ctx->launches;
-  if (g.trans_a) return g.trans_b ? direct_launch<true, false>(ctx, p, stream) : direct_launch<true, true>(ctx, p, stream);
-  return g.trans_b ? direct_launch<false, false>(ctx, p, stream) : direct_launch<false, true>(ctx, p, stream);
+  if (g.mode == B200_MODE_FP32_3XFP16) return direct_launch<true>(ctx, p, g.trans_a != 0, g.trans_b == 0, cols, stream);
+  return direct_launch<false>(ctx, p, g.trans_a != 0, g.trans_b == 0, cols, stream);
 }
 
 }  // namespace b200

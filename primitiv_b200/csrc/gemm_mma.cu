@@ -65,7 +65,7 @@ constexpr uint32_t kTileM[] = {128, 128, 128, 64, 128, 128}, kTileN[] = {8, 16, 
 // `ends` us besides, two CTAs of the small tiles and one of the large ones run at full speed on an SM, and
 // adding up a split costs 1.8 us.  Within 6 % of the best choice on average.
 MmaChoice choose(const b200_ctx *ctx, const GemmArgs &g, const MmaProblem &p) {
-  static const double kStep[3][6] = {{0.40, 0.48, 0.54, 0.59, 0.60, 0.95}, {0.52, 0.55, 0.60, 0.66, 0.70, 0.95}, {0.73, 0.81, 0.91, 1.0, 1.1, 0.0}};
+  static const double kStep[3][6] = {{0.40, 0.48, 0.54, 0.59, 0.60, 0.95}, {0.52, 0.55, 0.60, 0.66, 0.70, 0.95}, {0.75, 0.86, 1.0, 1.15, 1.25, 0.0}};
   static const double kEnds[3][6] = {{1.8, 2.0, 2.5, 2.1, 3.0, 4.4}, {2.0, 2.2, 2.9, 2.4, 3.3, 5.0}, {2.2, 2.4, 3.2, 2.7, 4.2, 0.0}};
   MmaChoice best{kTile64x64, 1, 1e30};
   for (int t = 0; t < 6; ++t) {
@@ -77,7 +77,9 @@ MmaChoice choose(const b200_ctx *ctx, const GemmArgs &g, const MmaProblem &p) {
     const double tiles = static_cast<double>((p.a.mn + kTileM[t] - 1) / kTileM[t]) * ((p.b.mn + kTileN[t] - 1) / kTileN[t]) * g.groups;
     const double room = ctx->sm_count * (t <= kTile64x64 ? 2.0 : 1.0);
     for (uint32_t s = 1; s <= 8u && s <= p.kt; s *= 2u) {
-      const double waves = tiles * s / room, load = waves > 1.0 ? waves : 1.0;
+      double waves = tiles * s / room;
+      if (p.kind == kMmaFp32) waves = static_cast<double>(static_cast<uint64_t>(waves + 0.999));   // (bound by arithmetic: a last wave costs a whole one)
+      const double load = waves > 1.0 ? waves : 1.0;
       const double us = load * (static_cast<double>((p.kt + s - 1) / s) * step + kEnds[p.kind][t]) + (s > 1u ? 1.8 : 0.0);
       if (us < best.us) best = {t, s, us};
     }
@@ -108,6 +110,8 @@ bool make_map(const b200_ctx *ctx, const MmaOperand &o, uint32_t k, uint32_t gro
 }  // namespace
 
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g) {
+  // (half planes lose less than TF32 ones where the sum is that short, see gemm_direct_estimate)
+  if (g.mode == B200_MODE_FP32_3XFP16 && static_cast<uint64_t>(g.k) * g.red < 64u && !tiny_or_thin(g)) return 1e30;
   const MmaProblem p = describe(g);
   // (the fixed part was fitted with the rest: `ends` has it)
   return choose(ctx, g, p).us + 0.5;
@@ -139,10 +143,10 @@ int gemm_mma(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream) {
     if (!make_map(ctx, q.a, g.k, g.groups, g.red, q.es, kTileM[c.tile], &p.map_a, &p.a_gmul, &p.a_rmul) ||
         !make_map(ctx, q.b, g.k, g.groups, g.red, q.es, kTileN[c.tile], &p.map_b, &p.b_gmul, &p.b_rmul))
       return B200_ERR_DRIVER;
-  } else {
-    p.A = q.a.ptr; p.lda = q.a.ld; p.a_gs = q.a.gs; p.a_rs = q.a.rs;
-    p.B = q.b.ptr; p.ldb = q.b.ld; p.b_gs = q.b.gs; p.b_rs = q.b.rs;
   }
+  p.A = q.a.ptr; p.lda = q.a.ld; p.a_gs = q.a.gs; p.a_rs = q.a.rs;
+  p.B = q.b.ptr; p.ldb = q.b.ld; p.b_gs = q.b.gs; p.b_rs = q.b.rs;
+  p.mend = q.kind == kMmaFp32 && tiny_or_thin(g) ? 1u : 0u;
   p.tiles_m = (p.m + kTileM[c.tile] - 1) / kTileM[c.tile];
   p.tiles_n = (p.n + kTileN[c.tile] - 1) / kTileN[c.tile];
   p.kb = q.kb;

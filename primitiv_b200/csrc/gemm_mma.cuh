@@ -9,9 +9,9 @@
 // to add the slices of a split contraction.  A product of a few microseconds is all ends.  Here
 //   - operands are fetched as they lie: with TMA where its alignment rules allow (one thread issues a
 //     k-tile), else with 4-byte cp.async, or single elements for halves on odd addresses;
-//   - the fp32 modes split x = hi + lo in registers, with the same arithmetic as the planes of
-//     pack.cu (hi = rn_tf32(x); the correction passes take bf16(x) and bf16(x - hi)), so nothing is
-//     written or read twice;
+//   - the fp32 modes split x = hi + lo in registers, both in TF32, so nothing is written or read twice.
+//     The smallest came from the CUDA cores, and their sums have to stay as good: with bf16 corrections, as
+//     the planes of pack.cu have them, 48 x 336 x 88 was off by 7.9e-7 where those had 1.7e-7;
 //   - a contraction is cut over the CTAs of a cluster, which add their tiles through distributed
 //     shared memory in rank order: one launch, no scratch, the same bits every run;
 //   - tiles go down to 128 x 8, so a handful of columns against a large matrix streams that matrix
@@ -28,11 +28,11 @@
 // MN-major floats, under the pattern on 32-byte units.
 //
 // The tensor core truncates when it adds into its accumulator (see gemm_tc.cu); the fp32 modes
-// therefore promote their accumulators to a second set of registers every kPromote elements of k.
+// therefore promote their accumulators to a second set of registers after every k-tile, and keep the small
+// terms out of them.
 #ifndef PRIMITIV_B200_CSRC_GEMM_MMA_CUH_
 #define PRIMITIV_B200_CSRC_GEMM_MMA_CUH_
 
-#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <atomic>
@@ -144,10 +144,6 @@ __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], c
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
 __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
   asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
@@ -231,31 +227,14 @@ __device__ __forceinline__ uint32_t nearest_tf32(uint32_t u) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(v) : "f"(__uint_as_float(u)));
   return v;
 }
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t *>(&v);
-}
-
-// Two k-steps (16 floats) of a fragment, split: x[s] = the fragment of step s.  hi[s] is x[s] in TF32; the
-// bf16 fragments of all 16 pair the two values a lane holds of each step, in the same way for A and for
-// B: the order of k inside a contraction is free.
+// The fp32 modes' fragments: x = hi + lo, both TF32.
 template <int N>
-__device__ __forceinline__ void split_fp32(const uint32_t (&x0)[N], const uint32_t (&x1)[N], uint32_t (&hi0)[N], uint32_t (&hi1)[N],
-                                           uint32_t (&h8)[N], uint32_t (&l8)[N]) {
-  constexpr int kHalfN = N / 2;   // registers [0, N/2) are the low half of k, [N/2, N) the high half
+__device__ __forceinline__ void split_fp32(uint32_t (&x)[N], uint32_t (&lo)[N]) {
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    hi0[i] = round_tf32(x0[i]);
-    hi1[i] = round_tf32(x1[i]);
-  }
-#pragma unroll
-  for (int i = 0; i < kHalfN; ++i) {
-    const float a0 = __uint_as_float(x0[i]), a1 = __uint_as_float(x0[i + kHalfN]);
-    const float b0 = __uint_as_float(x1[i]), b1 = __uint_as_float(x1[i + kHalfN]);
-    h8[i] = pack_bf16(a0, a1);
-    h8[i + kHalfN] = pack_bf16(b0, b1);
-    l8[i] = pack_bf16(a0 - __uint_as_float(hi0[i]), a1 - __uint_as_float(hi0[i + kHalfN]));
-    l8[i + kHalfN] = pack_bf16(b0 - __uint_as_float(hi1[i]), b1 - __uint_as_float(hi1[i + kHalfN]));
+    const uint32_t hi = round_tf32(x[i]);
+    lo[i] = round_tf32(__float_as_uint(__uint_as_float(x[i]) - __uint_as_float(hi)));
+    x[i] = hi;
   }
 }
 
@@ -288,7 +267,26 @@ __device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-constexpr uint32_t kPromote = 128;   // elements of k between promotions of the fp32 modes' accumulators
+// An infinite operand makes x - hi a nan, or meets the zero it left of another one.  Tiny and thin products, which are the
+// CUDA cores' by their numerics, sum an element that is not finite again as those do.
+template <bool KA, bool KB>
+__device__ __noinline__ float plain_sum(const MmaParams &p, uint32_t g, uint32_t i, uint32_t j) {
+  float v = 0.f;
+  for (uint32_t r = 0; r < p.kt / p.kb; ++r) {
+    const float *a = static_cast<const float *>(p.A) + g * p.a_gs + r * p.a_rs + i * (KA ? p.lda : 1ull);
+    const float *b = static_cast<const float *>(p.B) + g * p.b_gs + r * p.b_rs + j * (KB ? p.ldb : 1ull);
+    for (uint32_t k = 0; k < p.k; ++k) v = fmaf(a[k * (KA ? 1ull : p.lda)], b[k * (KB ? 1ull : p.ldb)], v);
+  }
+  return v;
+}
+template <bool KA, bool KB>
+__device__ __forceinline__ void mend(float4 &v, const MmaParams &p, uint32_t g, uint32_t i, uint32_t j) {
+  if (!p.mend || fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) <= 3e38f) return;
+  if (!(fabsf(v.x) <= 3e38f)) v.x = plain_sum<KA, KB>(p, g, i, j);
+  if (!(fabsf(v.y) <= 3e38f) && i + 1u < p.m) v.y = plain_sum<KA, KB>(p, g, i + 1u, j);
+  if (!(fabsf(v.z) <= 3e38f) && i + 2u < p.m) v.z = plain_sum<KA, KB>(p, g, i + 2u, j);
+  if (!(fabsf(v.w) <= 3e38f) && i + 3u < p.m) v.w = plain_sum<KA, KB>(p, g, i + 3u, j);
+}
 
 template <int KIND, int BM, int BN, int WM, int WN, int STAGES>
 struct MmaTile {
@@ -334,7 +332,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
   }
 
   float acc[MT][NB][4];
-  float sum[KIND == kMmaFp32 ? MT : 1][KIND == kMmaFp32 ? NB : 1][4];
+  float sum[KIND == kMmaFp32 ? MT : 1][KIND == kMmaFp32 ? NB : 1][4], cor[KIND == kMmaFp32 ? MT : 1][KIND == kMmaFp32 ? NB : 1][4];
 #pragma unroll
   for (int i = 0; i < MT; ++i)
 #pragma unroll
@@ -342,7 +340,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         acc[i][j][q] = 0.f;
-        if constexpr (KIND == kMmaFp32) sum[i][j][q] = 0.f;
+        if constexpr (KIND == kMmaFp32) sum[i][j][q] = cor[i][j][q] = 0.f;
       }
 
   pdl_wait_previous();
@@ -390,53 +388,40 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
     }
     if constexpr (KIND == kMmaFp32) {
 #pragma unroll
-      for (uint32_t ks = 0; ks < 4u; ks += 2u) {
-        uint32_t bh0[NB][2], bh1[NB][2], b8[NB][2], bl[NB][2];
-        {
-          uint32_t x0[NB][2], x1[NB][2];
-          frag_b<KB, kES, BN, NB>(x0, sb, wn, ks, lane);
-          frag_b<KB, kES, BN, NB>(x1, sb, wn, ks + 1u, lane);
+      for (uint32_t ks = 0; ks < 4u; ++ks) {
+        uint32_t bh[NB][2], bl[NB][2], ah[MT][4], al[MT][4];
+        frag_b<KB, kES, BN, NB>(bh, sb, wn, ks, lane);
 #pragma unroll
-          for (int j = 0; j < NB; ++j) split_fp32<2>(x0[j], x1[j], bh0[j], bh1[j], b8[j], bl[j]);
-        }
-        uint32_t ah0[MT][4], ah1[MT][4], a8[MT][4], al[MT][4];
+        for (int j = 0; j < NB; ++j) split_fp32<2>(bh[j], bl[j]);
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
-          uint32_t x0[4], x1[4];
-          frag_a<KA, kES, BM>(x0, sa, wm + i * 16u, ks, lane);
-          frag_a<KA, kES, BM>(x1, sa, wm + i * 16u, ks + 1u, lane);
-          split_fp32<4>(x0, x1, ah0[i], ah1[i], a8[i], al[i]);
+          frag_a<KA, kES, BM>(ah[i], sa, wm + i * 16u, ks, lane);
+          split_fp32<4>(ah[i], al[i]);
         }
-        // small terms first; one pass over all accumulators at a time, so that neighbouring instructions
-        // do not wait for each other's sums
+        // one pass over all accumulators at a time, so that neighbouring instructions do not wait for each
+        // other's sums
 #pragma unroll
         for (int i = 0; i < MT; ++i)
 #pragma unroll
-          for (int j = 0; j < NB; ++j) mma_bf16(acc[i][j], al[i], b8[j]);
+          for (int j = 0; j < NB; ++j) mma_tf32(cor[i][j], al[i], bh[j]);
 #pragma unroll
         for (int i = 0; i < MT; ++i)
 #pragma unroll
-          for (int j = 0; j < NB; ++j) mma_bf16(acc[i][j], a8[i], bl[j]);
+          for (int j = 0; j < NB; ++j) mma_tf32(acc[i][j], ah[i], bh[j]);
 #pragma unroll
         for (int i = 0; i < MT; ++i)
 #pragma unroll
-          for (int j = 0; j < NB; ++j) mma_tf32(acc[i][j], ah0[i], bh0[j]);
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-          for (int j = 0; j < NB; ++j) mma_tf32(acc[i][j], ah1[i], bh1[j]);
+          for (int j = 0; j < NB; ++j) mma_tf32(cor[i][j], ah[i], bl[j]);
       }
-      if ((it - (STAGES - 2u)) % (kPromote / Tile::kBK) == 0u) {
 #pragma unroll
-        for (int i = 0; i < MT; ++i)
+      for (int i = 0; i < MT; ++i)
 #pragma unroll
-          for (int j = 0; j < NB; ++j)
+        for (int j = 0; j < NB; ++j)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              sum[i][j][q] += acc[i][j][q];
-              acc[i][j][q] = 0.f;
-            }
-      }
+          for (int q = 0; q < 4; ++q) {
+            sum[i][j][q] += acc[i][j][q];
+            acc[i][j][q] = 0.f;
+          }
     } else {
 #pragma unroll
       for (uint32_t ks = 0; ks < 4u; ++ks) {
@@ -481,7 +466,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
         for (int q = 0; q < 4; ++q) {
           const uint32_t mm = wm + i * 16u + gq + ((q >> 1) << 3), nn = wn + j * 8u + t * 2u + (q & 1);
           float v = acc[i][j][q];
-          if constexpr (KIND == kMmaFp32) v += sum[i][j][q];
+          if constexpr (KIND == kMmaFp32) v = sum[i][j][q] + cor[i][j][q];
           out[nn * Tile::kPitch + mm] = v;
         }
   }
@@ -510,6 +495,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
       } else {
         v = *reinterpret_cast<const float4 *>(out + nn * Tile::kPitch + mm);
       }
+      if constexpr (KIND == kMmaFp32) mend<KA, KB>(v, p, g, gm, gn);
       T *c = C + gm + gn * p.c_n;
       const bool whole = gm + 4u <= p.m && (reinterpret_cast<unsigned long long>(c) & (4u * kES - 1u)) == 0;
       if (whole) {
@@ -553,6 +539,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
       } else {
         v = *reinterpret_cast<const float4 *>(out + nn * Tile::kPitch + mm);
       }
+      if constexpr (KIND == kMmaFp32) mend<KA, KB>(v, p, g, gm, gn);
       T *c = C + gm * p.c_m + gn;
       const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll

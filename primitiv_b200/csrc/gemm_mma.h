@@ -27,6 +27,7 @@ struct alignas(64) MmaParams {
   uint32_t a_gmul, a_rmul, b_gmul, b_rmul;   // matrix (g, r) of an operand is number g * gmul + r * rmul of its map
   uint32_t load;
   uint32_t accumulate;
+  uint32_t mend;                 // elements that are not finite are summed again, as the CUDA cores would
   int *status;
 };
 

@@ -788,6 +788,7 @@ TileChoice choose_tile(const b200_ctx *ctx, const GemmArgs &g, const TileCost &c
                        bool may_split) {
   const double clocks_per_us = 1850.0;
   static const struct { uint32_t ctas, bn; } kShapes[] = {{2, 256}, {1, 256}, {1, 128}, {1, 64}};
+  const uint32_t fixed = may_split ? gemm_fixed_slices(ctx, g) : 0u;
   TileChoice best{1, 64, 1, 1e30};
   for (const auto &sh : kShapes) {
     if (sh.bn > 64u && sh.bn / 2u >= g.n) continue;   // half the columns or more would be padding
@@ -800,7 +801,8 @@ TileChoice choose_tile(const b200_ctx *ctx, const GemmArgs &g, const TileCost &c
     const double per_kblock = load > mma ? load : mma;
     const uint32_t stages_k = (kblocks + kblocks_per_stage - 1) / kblocks_per_stage;
     // (a split is at least two pipeline stages, and never more work items than one wave)
-    for (uint32_t s = 1; s <= 64u && (s == 1u || (may_split && s * 2u <= stages_k && tiles * s <= units)); s += s < 4u ? 1u : s / 4u) {
+    for (uint32_t s = fixed ? fixed : 1u; s <= 64u && (s == 1u || s == fixed || (may_split && s * 2u <= stages_k && tiles * s <= units));
+         s += fixed ? 64u : s < 4u ? 1u : s / 4u) {
       const double kb = static_cast<double>((stages_k + s - 1) / s) * kblocks_per_stage * g.red;
       const double waves = static_cast<double>(static_cast<uint64_t>((tiles * s + units - 1) / units));
       const double main = kb * per_kblock + 1.0, write = 0.0125 * sh.bn;
@@ -1215,8 +1217,12 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
     p.mix_boxes = nb;
   }
   p.passes = passes;
-  const bool chunked = passes == 3 && static_cast<uint64_t>(g.red) * p.kblocks > kChunkKBlocks;
-  p.chunk_kblocks = chunked ? kChunkKBlocks : g.red * p.kblocks;
+  // (a longer chunk truncates more: products of one wave, whose slices are cut as speed has it, take chunks of half
+  // the length and are no less precise for it, however long a slice is)
+  const bool one_wave = may_split && launch_tiles <= static_cast<uint64_t>(ctx->sm_count) / ctas;
+  const uint32_t chunk_len = one_wave && !gemm_fixed_slices(ctx, g) ? kChunkKBlocks / 2u : kChunkKBlocks;
+  const bool chunked = passes == 3 && static_cast<uint64_t>(g.red) * p.kblocks > chunk_len;
+  p.chunk_kblocks = chunked ? chunk_len : g.red * p.kblocks;
   p.accumulate = g.accumulate ? 1u : 0u;
   p.out_half = half_store ? 1u : 0u;
   p.kind_f16 = f16 ? 1u : 0u;
@@ -1375,8 +1381,26 @@ bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g) {
   return direct_ok(a.ptr, a.ld, a.batch_stride, a.nbatch, eb) && direct_ok(b.ptr, b.ld, b.batch_stride, b.nbatch, eb);
 }
 
+// The fp32 mode sums a contraction of up to 1024 terms in one order, given by the sizes alone: the same bits whether
+// the operands come in planes or are split by the kernel, whatever the tile.  Activations pass or block a
+// gradient by their sign, and one value near zero that falls to the other side moves the weight gradient of an
+// 800-wide layer over 200 items by 0.25 %: a choice of kernel or tile should not do that.  The order is that of
+// 256-row, 256-column pair tiles with slices of four k-blocks or more for the pairs they leave idle.
+uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g) {
+  if (g.mode != B200_MODE_FP32_3XTF32 || g.red != 1u || g.k > 1024u) return 0u;
+  const uint32_t kb = (g.k + 31u) / 32u;
+  const uint32_t bn = g.n > 128u ? 256u : g.n > 64u ? 128u : 64u, rows = bn >= 128u && g.m > kBM ? 2u * kBM : kBM;
+  const uint64_t tiles = static_cast<uint64_t>((g.m + rows - 1) / rows) * ((g.n + bn - 1) / bn) * g.groups;
+  const uint64_t units = static_cast<uint64_t>(ctx->sm_count) * kBM / rows;
+  if (ctx->split_policy == 1 || kb < 16u || tiles * 2u > units) return 1u;
+  uint64_t want = units / tiles;
+  if (want > kb / 4u) want = kb / 4u;
+  const uint32_t per = (kb + static_cast<uint32_t>(want) - 1u) / static_cast<uint32_t>(want);
+  return (kb + per - 1u) / per;
+}
+
 double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g) {
-  if (!gemm_tc_eligible(ctx, g) || (g.mode == B200_MODE_TF32 && tiny_or_thin(g))) return 1e30;
+  if (!gemm_tc_eligible(ctx, g) || (g.mode != B200_MODE_FP16 && tiny_or_thin(g))) return 1e30;
   OperandView a, b;
   operand_views(g, &a, &b);
   const bool half = g.mode == B200_MODE_FP16 || g.mode == B200_MODE_FP32_3XFP16;

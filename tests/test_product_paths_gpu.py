@@ -78,3 +78,44 @@ def test_padded_lines_are_shared_inside_one_backward_call(ctx, mode):
     want_b = torch.einsum("nji,nki->nkj", a64, gy64)
     for got, want in ((ga, want_a), (gb, want_b)):
         assert (got.double().view_as(want) - want).norm() <= TOL[mode] * want.norm()
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+def test_sums_of_the_fp32_mode_do_not_depend_on_the_kernel(ctx, layout):
+    """Up to 1024 terms are summed in one order: both tcgen05 kernels give the same bits, with tiles of 32, 64
+    and 96 columns, with and without slices, at ragged ends of all three extents."""
+    ta, tb = (int(c == "t") for c in layout)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(11)
+    for m, n, k, groups in ((800, 200, 784, 1), (256, 1024, 256, 1), (129, 33, 1024, 1), (515, 97, 999, 1), (1000, 300, 515, 2), (64, 70, 40, 3)):
+        a, b = (torch.randn(groups * s, device="cuda", generator=gen) for s in (m * k, k * n))
+        got = []
+        for path in (2, 5):
+            c = torch.empty(groups * m * n, device="cuda")
+            ctx.gemm(MODES["3xtf32"], ta, tb, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, groups, 1, m * k, 0, k * n, 0, m * n, False, path)
+            got.append(c)
+        assert ctx.status_poll() == 0
+        assert torch.equal(*got), (m, n, k, groups)
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+def test_tiny_products_carry_infinities_and_nans_as_fp32_does(ctx, layout):
+    """An infinite term is an infinite sum (not the nan of inf - inf or inf * 0 inside a split), a nan a nan."""
+    ta, tb = (int(c == "t") for c in layout)
+    for m, n, k in ((48, 72, 96), (9, 300, 50), (200, 8, 1000)):
+        a, b = torch.ones(m * k, device="cuda"), torch.full((k * n,), 0.5, device="cuda")
+        at = lambda i, p: i * k + p if ta else p * m + i
+        a[at(0, 3)], a[at(1, 5)], a[at(2, 0)] = float("inf"), float("-inf"), float("nan")
+        a[at(3, 1)], a[at(3, 2)] = float("inf"), float("-inf")
+        a[at(4, 7)] = 3.4e38
+        want = product(a, b, ta, tb, m, n, k)
+        for mode in ("3xtf32", "tf32", "3xfp16"):
+            for path in (0, 4):
+                c = torch.empty(m * n, device="cuda")
+                ctx.gemm(MODES[mode], ta, tb, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, 1, 1, 0, 0, 0, 0, 0, False, path)
+                assert ctx.status_poll() == 0
+                got, fine = c.view(n, m), want.view(n, m)
+                assert torch.equal(torch.isnan(got), torch.isnan(fine)), (m, n, k, mode, path)
+                finite = torch.isfinite(fine)
+                assert torch.equal(got[~finite & ~torch.isnan(fine)], fine[~finite & ~torch.isnan(fine)])
+                assert ((got - fine)[finite].abs() <= 1e-5 * fine[finite].abs()).all()
