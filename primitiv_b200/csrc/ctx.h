@@ -136,7 +136,7 @@ struct b200_ctx {
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
   std::size_t smem_optin = 0;
-  int cluster_room[9] = {};      // clusters of 1 to 8 CTAs that run at a time with an SM to each CTA
+  int cluster_room[9] = {}, cluster_room_two[9] = {};   // clusters of 1 to 8 CTAs that run at a time, one or two CTAs to an SM
   b200::Pool pool;
   // Status word of the bounded device-side waits.  It lives in pinned host memory that the
   // GPU writes through a mapped alias (d_status): a kernel whose wait ran out stores its code
@@ -237,7 +237,7 @@ int gemm_skinny(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 int gemm_mma(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // fp32 modes, tcgen05 fed by the kernel's own loads: any shape, any alignment (gemm_direct.cu).
 int gemm_direct(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
-int gemm_direct_init(b200_ctx *ctx);   // fills cluster_room
+int gemm_direct_init(b200_ctx *ctx);   // fills cluster_room and cluster_room_two
 // tcgen05 path.  tc_eligible() says whether the operands meet TMA's alignment rules.
 bool gemm_tc_eligible(const b200_ctx *ctx, const GemmArgs &g);
 int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);

@@ -512,20 +512,22 @@ int gemm_direct_init(b200_ctx *ctx) {
   auto kernel = gemm_direct_kernel<true, true, 64u, false>;
   constexpr uint32_t kSmem = kDirectSmem<true, true, 64u>;
   B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
-  ctx->cluster_room[1] = ctx->sm_count;
-  for (unsigned s = 2; s <= 8u; ++s) {
+  for (unsigned s = 1; s <= 8u; ++s) {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = s;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.gridDim = dim3(s);
-    cfg.blockDim = dim3(kFeedThreads + 32u);
-    cfg.dynamicSmemBytes = kSmem;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    B200_CUDA_TRY(cudaOccupancyMaxActiveClusters(&ctx->cluster_room[s], kernel, &cfg));
-    if (ctx->cluster_room[s] < 1) ctx->cluster_room[s] = 1;
+    for (int two = 0; two < 2; ++two) {
+      int *room = two ? &ctx->cluster_room_two[s] : &ctx->cluster_room[s];
+      cfg.blockDim = dim3(two ? 128u : kFeedThreads + 32u);   // what the kernels of gemm_mma.cuh that share an SM have
+      cfg.dynamicSmemBytes = two ? 104u * 1024u : kSmem;
+      B200_CUDA_TRY(cudaOccupancyMaxActiveClusters(room, kernel, &cfg));
+      if (*room < 1) *room = 1;
+    }
   }
   return B200_OK;
 }

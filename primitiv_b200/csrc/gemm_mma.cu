@@ -75,9 +75,12 @@ MmaChoice choose(const b200_ctx *ctx, const GemmArgs &g, const MmaProblem &p) {
     if (p.load == kMmaWord && step < 1.8) step = 1.8;     // narrow copies bound a k-tile instead
     if (p.load == kMmaSingle && step < 6.0) step = 6.0;
     const double tiles = static_cast<double>((p.a.mn + kTileM[t] - 1) / kTileM[t]) * ((p.b.mn + kTileN[t] - 1) / kTileN[t]) * g.groups;
-    const double room = ctx->sm_count * (t <= kTile64x64 ? 2.0 : 1.0);
-    for (uint32_t s = 1; s <= 8u && s <= p.kt; s *= 2u) {
-      double waves = tiles * s / room;
+    const int *clusters = t <= kTile64x64 ? ctx->cluster_room_two : ctx->cluster_room;
+    for (uint32_t s = 1; s <= 8u && s <= p.kt; ++s) {
+      // (a cluster has to fit a GPC: 32 clusters of eight, two CTAs to an SM, do not run at once, nor does half of
+      // one more count; four 4096-wide layers of halves over 8 columns spent twice the time so)
+      double waves = tiles / clusters[s];
+      if (s > 1u) waves = static_cast<double>(static_cast<uint64_t>(waves + 0.999));
       if (p.kind == kMmaFp32) waves = static_cast<double>(static_cast<uint64_t>(waves + 0.999));   // (bound by arithmetic: a last wave costs a whole one)
       const double load = waves > 1.0 ? waves : 1.0;
       const double us = load * (static_cast<double>((p.kt + s - 1) / s) * step + kEnds[p.kind][t]) + (s > 1u ? 1.8 : 0.0);
