@@ -193,22 +193,23 @@ __global__ void __launch_bounds__(kBlock) binary_bw_flat_kernel(const T *__restr
 // One operand is broadcast over the batch: its gradient is the sum over the batch of the
 // per-item terms (32 x 8 CTAs over volume x batch slices, see batch_sum_tile_kernel); the
 // batched operand's gradient is updated in place on the way.
-template <typename T, int OP>
+template <typename T, int OP, unsigned kLanes>
 __global__ void __launch_bounds__(256) binary_bw_mixed_kernel(const T *__restrict__ a, const T *__restrict__ b,
                                                               const T *__restrict__ y, const T *__restrict__ gy,
                                                               T *ga, T *gb, float *partial, u64 volume,
                                                               uint32_t batch, uint32_t slice_len, int a_batched,
                                                               int acc_batched, int acc_summed) {
   pdl_enter();
-  __shared__ float buf[kSumLanes][32];
+  constexpr unsigned kX = 256u / kLanes;
+  __shared__ float buf[kLanes][kX];
   T *g_batched = a_batched ? ga : gb, *g_summed = a_batched ? gb : ga;
-  for (u64 tile = blockIdx.x; tile * 32ull < volume; tile += gridDim.x) {
-    const u64 i = tile * 32ull + threadIdx.x;
+  for (u64 tile = blockIdx.x; tile * kX < volume; tile += gridDim.x) {
+    const u64 i = tile * kX + threadIdx.x;
     const uint32_t lo = blockIdx.y * slice_len;
     const uint32_t hi = lo + slice_len < batch ? lo + slice_len : batch;
     float v = 0.f;
     if (i < volume) {
-      for (uint32_t n = lo + threadIdx.y; n < hi; n += kSumLanes) {
+      for (uint32_t n = lo + threadIdx.y; n < hi; n += kLanes) {
         const u64 e = static_cast<u64>(n) * volume + i;
         float da, db;
         binary_d<OP>(ld(a, a_batched ? e : i), ld(b, a_batched ? i : e), ld(y, e), ld(gy, e), da, db);
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(256) binary_bw_mixed_kernel(const T *__restric
         v += a_batched ? db : da;
       }
     }
-    const float t = combine_batch_lanes(v, buf);
+    const float t = combine_batch_lanes<kLanes>(v, buf);
     if (threadIdx.y == 0 && i < volume) {
       if (gridDim.y == 1) st(g_summed, i, (acc_summed ? ld(g_summed, i) : 0.f) + t);
       else partial[static_cast<u64>(blockIdx.y) * volume + i] = t;
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(256) binary_bw_mixed_kernel(const T *__restric
 // the first of them is stored, so that the stores (which may alias the loads as far as the
 // compiler knows) do not put one memory latency between every two items.  Only the operands the
 // derivative needs are read at all (none for + and -).
-template <typename T, int OP>
+template <typename T, int OP, unsigned kLanes>
 __global__ void __launch_bounds__(256) binary_bw_mixed_vec_kernel(const T *__restrict__ a, const T *__restrict__ b,
                                                                   const T *__restrict__ y, const T *__restrict__ gy,
                                                                   T *ga, T *gb, float *partial, u64 volume,
@@ -237,16 +238,16 @@ __global__ void __launch_bounds__(256) binary_bw_mixed_vec_kernel(const T *__res
                                                                   int acc_batched, int acc_summed) {
   pdl_enter();
   constexpr int N = Vec<T>::N;
-  constexpr unsigned U = 4;
+  constexpr unsigned U = 4, kX = 256u / kLanes;
   constexpr bool kNeedA = OP == B200_OP_MULTIPLY || OP == B200_OP_POW;                        // db or da reads a
   constexpr bool kNeedB = OP == B200_OP_MULTIPLY || OP == B200_OP_DIVIDE || OP == B200_OP_POW;
   constexpr bool kNeedY = OP == B200_OP_DIVIDE || OP == B200_OP_POW;
-  __shared__ float buf[kSumLanes][32 * N];
+  __shared__ float buf[kLanes][kX * N];
   T *g_batched = a_batched ? ga : gb, *g_summed = a_batched ? gb : ga;
   const T *op_batched = a_batched ? a : b, *op_shared = a_batched ? b : a;
   const bool need_batched = a_batched ? kNeedA : kNeedB, need_shared = a_batched ? kNeedB : kNeedA;
-  for (u64 tile = blockIdx.x; tile * (32ull * N) < volume; tile += gridDim.x) {
-    const u64 i = (tile * 32ull + threadIdx.x) * N;
+  for (u64 tile = blockIdx.x; tile * (kX * N) < volume; tile += gridDim.x) {
+    const u64 i = (tile * kX + threadIdx.x) * N;
     const uint32_t lo = blockIdx.y * slice_len;
     const uint32_t hi = lo + slice_len < batch ? lo + slice_len : batch;
     float v[N];
@@ -256,15 +257,15 @@ __global__ void __launch_bounds__(256) binary_bw_mixed_vec_kernel(const T *__res
       Vec<T> vs;
       vs.raw = {};
       if (need_shared) vs.load(op_shared + i);
-      for (uint32_t n = lo + threadIdx.y; n < hi; n += kSumLanes * U) {
+      for (uint32_t n = lo + threadIdx.y; n < hi; n += kLanes * U) {
         Vec<T> vgy[U], vop[U], vy[U], vold[U];
 #pragma unroll
         for (unsigned u = 0; u < U; ++u) {
           vop[u].raw = {};
           vy[u].raw = {};
           vold[u].raw = {};
-          if (n + u * kSumLanes < hi) {
-            const u64 e = static_cast<u64>(n + u * kSumLanes) * volume + i;
+          if (n + u * kLanes < hi) {
+            const u64 e = static_cast<u64>(n + u * kLanes) * volume + i;
             vgy[u].load(gy + e);
             if (need_batched) vop[u].load(op_batched + e);
             if (kNeedY) vy[u].load(y + e);
@@ -273,8 +274,8 @@ __global__ void __launch_bounds__(256) binary_bw_mixed_vec_kernel(const T *__res
         }
 #pragma unroll
         for (unsigned u = 0; u < U; ++u) {
-          if (n + u * kSumLanes < hi) {
-            const u64 e = static_cast<u64>(n + u * kSumLanes) * volume + i;
+          if (n + u * kLanes < hi) {
+            const u64 e = static_cast<u64>(n + u * kLanes) * volume + i;
             Vec<T> out;
 #pragma unroll
             for (int j = 0; j < N; ++j) {
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(256) binary_bw_mixed_vec_kernel(const T *__res
         }
       }
     }
-    combine_batch_lanes_vec<N>(v, buf);
+    combine_batch_lanes_vec<N, kLanes>(v, buf);
     if (threadIdx.y == 0 && i < volume) {
 #pragma unroll
       for (int j = 0; j < N; ++j) {
@@ -458,19 +459,19 @@ int launch_binary_bw(b200_ctx *ctx, cudaStream_t s, int op, const void *a, const
     const int rc = ctx->pool.alloc(static_cast<size_t>(bs.slices) * volume * sizeof(float), &partial, nullptr);
     if (rc != B200_OK) return rc;
   }
-  const dim3 grid(bs.tiles, bs.slices), block(32, kSumLanes);
-  if (vec) {
-    switch (op) {
-#define X(OP) case OP: b200::launch(ctx, binary_bw_mixed_vec_kernel<T, OP>, dim3(grid), dim3(block), 0, s, 1u, pa, pb, py, pgy, pga, pgb, static_cast<float *>(partial), volume, batch, bs.slice_len, a_batched, a_batched ? acc_a : acc_b, a_batched ? acc_b : acc_a); break;
-      B200_BINARY_OPS(X)
+  const dim3 grid(bs.tiles, bs.slices), block = bs.many ? dim3(8, kSumManyLanes) : dim3(32, kSumLanes);
+  const auto run = [&](auto kernel) {
+    b200::launch(ctx, kernel, grid, block, 0, s, 1u, pa, pb, py, pgy, pga, pgb, static_cast<float *>(partial), volume, batch, bs.slice_len, a_batched,
+                 a_batched ? acc_a : acc_b, a_batched ? acc_b : acc_a);
+  };
+  switch (op) {
+#define X(OP)                                                                                                                          \
+  case OP:                                                                                                                             \
+    if (vec) run(bs.many ? binary_bw_mixed_vec_kernel<T, OP, kSumManyLanes> : binary_bw_mixed_vec_kernel<T, OP, kSumLanes>);            \
+    else run(bs.many ? binary_bw_mixed_kernel<T, OP, kSumManyLanes> : binary_bw_mixed_kernel<T, OP, kSumLanes>);                        \
+    break;
+    B200_BINARY_OPS(X)
 #undef X
-    }
-  } else {
-    switch (op) {
-#define X(OP) case OP: b200::launch(ctx, binary_bw_mixed_kernel<T, OP>, dim3(grid), dim3(block), 0, s, 1u, pa, pb, py, pgy, pga, pgb, static_cast<float *>(partial), volume, batch, bs.slice_len, a_batched, a_batched ? acc_a : acc_b, a_batched ? acc_b : acc_a); break;
-      B200_BINARY_OPS(X)
-#undef X
-    }
   }
   if (bs.slices > 1) {
     launch_batch_final<T>(ctx, s, static_cast<const float *>(partial), a_batched ? pgb : pga, volume, bs.slices, 1.f,

@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) slice_bw_sum_kernel(const T *__restrict__
     float v = 0.f;
     if (e < per_batch)
       for (uint32_t n = threadIdx.y; n < batch; n += kSumLanes) v += ld(gy, static_cast<u64>(n) * per_batch + e);
-    const float t = combine_batch_lanes(v, buf);
+    const float t = combine_batch_lanes<kSumLanes>(v, buf);
     if (threadIdx.y == 0 && e < per_batch) {
       const u64 r = e / span, j = e - r * span;
       const u64 d = off + r * skip + j;

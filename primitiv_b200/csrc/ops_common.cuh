@@ -58,17 +58,23 @@ inline unsigned grid_for(const b200_ctx *ctx, u64 work, unsigned block) {
 // slice, batch lane t adds items t, t + 8, ... in order and the 8 lanes are combined in lane
 // order; slices are combined in slice order by batch_final_kernel.  No atomics: the result is
 // the same bits on every run.
-constexpr unsigned kSumLanes = 8;
+//
+// A short batch is one slice, and a small volume then leaves the GPU to a few CTAs that walk it item after
+// item: 800 values x 200 items were 7 CTAs, 8.4 us of waiting.  Such sums take CTAs of 8 x 32 threads: four
+// times the CTAs, a quarter of the items per lane.
+constexpr unsigned kSumLanes = 8, kSumManyLanes = 32;
 
 struct BatchSlices {
   unsigned tiles;      // grid.x: volume / 32, rounded up
   unsigned slices;     // grid.y
   uint32_t slice_len;  // batch items per slice
+  bool many;           // CTAs of 8 x 32 threads
 };
 
 // tile_elems: consecutive elements of the volume per CTA (32, or 32 vectors of 4 / 8 in the vector forms)
 inline BatchSlices batch_slices(const b200_ctx *ctx, u64 volume, uint32_t batch, unsigned tile_elems = 32u) {
   BatchSlices r;
+  r.many = false;
   const u64 tiles = (volume + tile_elems - 1ull) / tile_elems;
   r.tiles = static_cast<unsigned>(tiles < 0x7fffffffull ? tiles : 0x7fffffffull);
   u64 want = (2ull * static_cast<u64>(ctx->sm_count) + tiles - 1) / tiles;  // about two CTAs per SM
@@ -79,17 +85,23 @@ inline BatchSlices batch_slices(const b200_ctx *ctx, u64 volume, uint32_t batch,
   if (want < 1) want = 1;
   r.slice_len = static_cast<uint32_t>((batch + want - 1) / want);
   r.slices = static_cast<unsigned>((batch + r.slice_len - 1) / r.slice_len);
+  // (half the SMs idle, and at least two items for most of the 32 lanes)
+  if (r.slices == 1u && batch >= 64u && tiles * 2ull <= static_cast<u64>(ctx->sm_count)) {
+    r.many = true;
+    r.tiles = static_cast<unsigned>((volume * 4ull + tile_elems - 1ull) / tile_elems);
+  }
   return r;
 }
 
-// Combines the 8 batch lanes of a CTA (lane order) and returns the total in batch lane 0.
-__device__ __forceinline__ float combine_batch_lanes(float v, float (*buf)[32]) {
+// Combines the batch lanes of a CTA (lane order) and returns the total in batch lane 0.
+template <unsigned kLanes>
+__device__ __forceinline__ float combine_batch_lanes(float v, float (*buf)[256u / kLanes]) {
   buf[threadIdx.y][threadIdx.x] = v;
   __syncthreads();
   float t = 0.f;
   if (threadIdx.y == 0) {
 #pragma unroll
-    for (unsigned l = 0; l < kSumLanes; ++l) t += buf[l][threadIdx.x];
+    for (unsigned l = 0; l < kLanes; ++l) t += buf[l][threadIdx.x];
   }
   __syncthreads();
   return t;
@@ -142,20 +154,21 @@ inline void launch_batch_final(b200_ctx *ctx, cudaStream_t s, const float *parti
 
 // y[i] = (accumulate ? y[i] : 0) + scale * sum_n x[n][i]; with more than one slice the CTA's
 // sum goes to partial[slice][i] instead.
-template <typename T>
+template <typename T, unsigned kLanes>
 __global__ void __launch_bounds__(256) batch_sum_tile_kernel(const T *__restrict__ x, T *y, float *partial,
                                                              u64 volume, uint32_t batch, uint32_t slice_len,
                                                              float scale, int accumulate) {
   pdl_enter();
-  __shared__ float buf[kSumLanes][32];
-  for (u64 tile = blockIdx.x; tile * 32ull < volume; tile += gridDim.x) {
-    const u64 i = tile * 32ull + threadIdx.x;
+  constexpr unsigned kX = 256u / kLanes;
+  __shared__ float buf[kLanes][kX];
+  for (u64 tile = blockIdx.x; tile * kX < volume; tile += gridDim.x) {
+    const u64 i = tile * kX + threadIdx.x;
     const uint32_t lo = blockIdx.y * slice_len;
     const uint32_t hi = lo + slice_len < batch ? lo + slice_len : batch;
     float v = 0.f;
     if (i < volume)
-      for (uint32_t n = lo + threadIdx.y; n < hi; n += kSumLanes) v += ld(x, static_cast<u64>(n) * volume + i);
-    const float t = combine_batch_lanes(v, buf);
+      for (uint32_t n = lo + threadIdx.y; n < hi; n += kLanes) v += ld(x, static_cast<u64>(n) * volume + i);
+    const float t = combine_batch_lanes<kLanes>(v, buf);
     if (threadIdx.y == 0 && i < volume) {
       if (gridDim.y == 1) st(y, i, (accumulate ? ld(y, i) : 0.f) + scale * t);
       else partial[static_cast<u64>(blockIdx.y) * volume + i] = t;
@@ -163,18 +176,33 @@ __global__ void __launch_bounds__(256) batch_sum_tile_kernel(const T *__restrict
   }
 }
 
-// Combines the 8 batch lanes of a CTA for the N values each thread holds (vector forms).
-template <int N>
-__device__ __forceinline__ void combine_batch_lanes_vec(float (&v)[N], float (*buf)[32 * N]) {
+// Combines the batch lanes of a CTA for the N values each thread holds (vector forms).
+template <int N, unsigned kLanes>
+__device__ __forceinline__ void combine_batch_lanes_vec(float (&v)[N], float (*buf)[256u / kLanes * N]) {
+  constexpr unsigned kWidth = 256u / kLanes * N;
 #pragma unroll
   for (int j = 0; j < N; ++j) buf[threadIdx.y][threadIdx.x * N + j] = v[j];
   __syncthreads();
-  if (threadIdx.y == 0) {
+  if constexpr (kWidth < 256u) {
+    // few columns of many lanes: a thread each
+    const unsigned t = threadIdx.y * blockDim.x + threadIdx.x;
+    if (t < kWidth) {
+      float sum = 0.f;
+#pragma unroll
+      for (unsigned l = 0; l < kLanes; ++l) sum += buf[l][t];
+      buf[0][t] = sum;
+    }
+    __syncthreads();
+    if (threadIdx.y == 0) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] = buf[0][threadIdx.x * N + j];
+    }
+  } else if (threadIdx.y == 0) {
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       float t = 0.f;
 #pragma unroll
-      for (unsigned l = 0; l < kSumLanes; ++l) t += buf[l][threadIdx.x * N + j];
+      for (unsigned l = 0; l < kLanes; ++l) t += buf[l][threadIdx.x * N + j];
       v[j] = t;
     }
   }
@@ -183,36 +211,36 @@ __device__ __forceinline__ void combine_batch_lanes_vec(float (&v)[N], float (*b
 
 // Vector form of batch_sum_tile_kernel (volume a multiple of the vector width, 16-byte aligned
 // arrays): a thread owns one 128-bit vector of the volume and keeps four items in flight.
-template <typename T>
+template <typename T, unsigned kLanes>
 __global__ void __launch_bounds__(256) batch_sum_tile_vec_kernel(const T *__restrict__ x, T *y, float *partial,
                                                                  u64 volume, uint32_t batch, uint32_t slice_len,
                                                                  float scale, int accumulate) {
   pdl_enter();
   constexpr int N = Vec<T>::N;
-  constexpr unsigned U = 4;
-  __shared__ float buf[kSumLanes][32 * N];
-  for (u64 tile = blockIdx.x; tile * (32ull * N) < volume; tile += gridDim.x) {
-    const u64 i = (tile * 32ull + threadIdx.x) * N;
+  constexpr unsigned U = 4, kX = 256u / kLanes;
+  __shared__ float buf[kLanes][kX * N];
+  for (u64 tile = blockIdx.x; tile * (kX * N) < volume; tile += gridDim.x) {
+    const u64 i = (tile * kX + threadIdx.x) * N;
     const uint32_t lo = blockIdx.y * slice_len;
     const uint32_t hi = lo + slice_len < batch ? lo + slice_len : batch;
     float v[N];
 #pragma unroll
     for (int j = 0; j < N; ++j) v[j] = 0.f;
     if (i < volume) {
-      for (uint32_t n = lo + threadIdx.y; n < hi; n += kSumLanes * U) {
+      for (uint32_t n = lo + threadIdx.y; n < hi; n += kLanes * U) {
         Vec<T> vx[U];
 #pragma unroll
         for (unsigned u = 0; u < U; ++u)
-          if (n + u * kSumLanes < hi) vx[u].load(x + static_cast<u64>(n + u * kSumLanes) * volume + i);
+          if (n + u * kLanes < hi) vx[u].load(x + static_cast<u64>(n + u * kLanes) * volume + i);
 #pragma unroll
         for (unsigned u = 0; u < U; ++u)
-          if (n + u * kSumLanes < hi) {
+          if (n + u * kLanes < hi) {
 #pragma unroll
             for (int j = 0; j < N; ++j) v[j] += vx[u].get(j);
           }
       }
     }
-    combine_batch_lanes_vec<N>(v, buf);
+    combine_batch_lanes_vec<N, kLanes>(v, buf);
     if (threadIdx.y == 0 && i < volume) {
 #pragma unroll
       for (int j = 0; j < N; ++j) {
@@ -235,12 +263,11 @@ int launch_batch_sum(b200_ctx *ctx, cudaStream_t s, const void *x, void *y, u64 
     const int rc = ctx->pool.alloc(static_cast<size_t>(bs.slices) * volume * sizeof(float), &partial, nullptr);
     if (rc != B200_OK) return rc;
   }
-  if (vec)
-    b200::launch(ctx, batch_sum_tile_vec_kernel<T>, dim3(bs.tiles, bs.slices), dim3(32, kSumLanes), 0, s, 1u, static_cast<const T *>(x), static_cast<T *>(y), static_cast<float *>(partial), volume, batch, bs.slice_len,
-        scale, accumulate);
-  else
-    b200::launch(ctx, batch_sum_tile_kernel<T>, dim3(bs.tiles, bs.slices), dim3(32, kSumLanes), 0, s, 1u, static_cast<const T *>(x), static_cast<T *>(y), static_cast<float *>(partial), volume, batch, bs.slice_len,
-        scale, accumulate);
+  const dim3 grid(bs.tiles, bs.slices), block = bs.many ? dim3(8, kSumManyLanes) : dim3(32, kSumLanes);
+  auto kernel = vec ? (bs.many ? batch_sum_tile_vec_kernel<T, kSumManyLanes> : batch_sum_tile_vec_kernel<T, kSumLanes>)
+                    : (bs.many ? batch_sum_tile_kernel<T, kSumManyLanes> : batch_sum_tile_kernel<T, kSumLanes>);
+  b200::launch(ctx, kernel, grid, block, 0, s, 1u, static_cast<const T *>(x), static_cast<T *>(y), static_cast<float *>(partial), volume, batch,
+               bs.slice_len, scale, accumulate);
   if (bs.slices > 1) {
     launch_batch_final<T>(ctx, s, static_cast<const float *>(partial), static_cast<T *>(y), volume, bs.slices, scale, accumulate);
     ctx->pool.free(partial);  // stream-ordered reuse
