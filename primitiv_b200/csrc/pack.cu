@@ -568,40 +568,80 @@ __global__ void __launch_bounds__(256) pack_mix_kernel(const float *__restrict__
   }
 }
 
-// Any dense source, line by line, lines padded to `pad` elements (a multiple of 8) in the planes and the
-// padding left as it is (TMA is given the true extents).  1 << shift lanes walk a line, two elements a
-// lane and step, four steps in flight.  Bound by memory; what it replaces for ragged sizes transposed every
-// operand through 32 x 32 tiles in shared memory, for one use.
+// Any dense source, lines padded to `pad` elements (a multiple of 8) in the planes; what ends up in the padding
+// does not matter (TMA is given the true extents).  A thread makes 16 bytes of the first plane (8 halves, 4 floats)
+// at a time, of kPadUnits lines at once; 1 << shift threads share a line.  Halves come as aligned words, shifted by one
+// half where the line starts on an odd one.  Bound by memory and, for a few thousand lines, by its latency: with a warp
+// walking each line two elements a lane and load, 12 x 131 lines of 765 halves took 6.3 us, now 4.3 (lines enough to fill
+// the GPU, 12 x 765 of 1021: 9.4 before and now).
+constexpr uint32_t kPadUnits = 4;
+
 template <int kKind, typename T>
 __global__ void __launch_bounds__(256) pad_lines_kernel(const T *__restrict__ src, void *__restrict__ p0, void *__restrict__ p1,
                                                         void *__restrict__ p2, uint32_t line, uint32_t pad,
                                                         unsigned long long lines, uint32_t shift) {
   pdl_enter();
+  constexpr uint32_t kWide = 16u / sizeof(T);
+  constexpr bool kHalf = sizeof(T) == 2;
   const uint32_t lanes = 1u << shift, lane = threadIdx.x & (lanes - 1u);
-  const unsigned long long step = (static_cast<unsigned long long>(gridDim.x) * 256u) >> shift;
-  for (unsigned long long l = (blockIdx.x * 256ull + threadIdx.x) >> shift; l < lines; l += step) {
-    const T *s = src + l * line;
-    const unsigned long long d = l * pad;
-    for (uint32_t e0 = lane * 2u; e0 < line; e0 += lanes * 8u) {
-      T x[4][2];
+  const unsigned long long step = (static_cast<unsigned long long>(gridDim.x) * 256u) >> shift, total = lines * line;
+  for (unsigned long long l0 = (blockIdx.x * 256ull + threadIdx.x) >> shift; l0 < lines; l0 += step * kPadUnits) {
+    for (uint32_t e = lane * kWide; e < line; e += lanes * kWide) {
+      // elements [g, g + kWide) of the source, past the end of the line too, where the array has them
+      const unsigned long long g0 = l0 * line + e;
+      unsigned long long l1 = l0 + (kPadUnits - 1u) * step;   // the last of these lines
+      while (l1 >= lines) l1 -= step;
+      const bool inside = g0 >= 1ull && l1 * line + e + kWide + 2u <= total;
+      uint32_t w[kPadUnits][5];
+      if (inside) {
 #pragma unroll
-      for (uint32_t u = 0; u < 4u; ++u) {
-        const uint32_t e = e0 + u * lanes * 2u;
-        x[u][0] = e < line ? s[e] : T(0.f);
-        x[u][1] = e + 1u < line ? s[e + 1u] : T(0.f);
+        for (uint32_t u = 0; u < kPadUnits; ++u) {
+          const unsigned long long l = l0 + u * step;
+          const uintptr_t at = reinterpret_cast<uintptr_t>(src + (l < lines ? l : l0) * line + e);
+          const uint32_t *q = reinterpret_cast<const uint32_t *>(at & ~static_cast<uintptr_t>(3));
+#pragma unroll
+          for (uint32_t i = 0; i < (kHalf ? 5u : 4u); ++i) w[u][i] = q[i];
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kPadUnits; ++u) {
+          if constexpr (kHalf) {
+            const unsigned long long l = l0 + u * step;
+            const uint32_t by = (reinterpret_cast<uintptr_t>(src + (l < lines ? l : l0) * line + e) & 2u) * 8u;
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i) w[u][i] = __funnelshift_r(w[u][i], w[u][i + 1u], by);
+          }
+        }
+      } else {   // the array's ends: element by element
+#pragma unroll
+        for (uint32_t u = 0; u < kPadUnits; ++u) {
+          const unsigned long long l = l0 + u * step, g = l * line + e;
+#pragma unroll
+          for (uint32_t i = 0; i < 4u; ++i) {
+            w[u][i] = 0u;
+            if constexpr (kHalf) {
+              const unsigned short *h = reinterpret_cast<const unsigned short *>(src);
+              if (l < lines && g + 2u * i < total) w[u][i] = h[g + 2u * i];
+              if (l < lines && g + 2u * i + 1u < total) w[u][i] |= static_cast<uint32_t>(h[g + 2u * i + 1u]) << 16;
+            } else {
+              if (l < lines && g + i < total) w[u][i] = reinterpret_cast<const uint32_t *>(src)[g + i];
+            }
+          }
+        }
       }
 #pragma unroll
-      for (uint32_t u = 0; u < 4u; ++u) {
-        const uint32_t e = e0 + u * lanes * 2u;
-        if (e >= line) break;
-        if constexpr (kKind == kPlanesHalf) {
-          reinterpret_cast<__half2 *>(p0)[(d + e) >> 1] = __halves2half2(x[u][0], x[u][1]);
+      for (uint32_t u = 0; u < kPadUnits; ++u) {
+        const unsigned long long l = l0 + u * step;
+        if (l >= lines) break;
+        const unsigned long long d = (l * pad + e) / kWide;
+        if constexpr (kHalf) {
+          reinterpret_cast<uint4 *>(p0)[d] = make_uint4(w[u][0], w[u][1], w[u][2], w[u][3]);
         } else {
-          const float2 h = make_float2(rn_tf32(x[u][0]), rn_tf32(x[u][1]));
-          reinterpret_cast<float2 *>(p0)[(d + e) >> 1] = h;
+          const float4 x = make_float4(__uint_as_float(w[u][0]), __uint_as_float(w[u][1]), __uint_as_float(w[u][2]), __uint_as_float(w[u][3]));
+          const float4 h = make_float4(rn_tf32(x.x), rn_tf32(x.y), rn_tf32(x.z), rn_tf32(x.w));
+          reinterpret_cast<float4 *>(p0)[d] = h;
           if constexpr (kKind == kPlanesMix) {
-            reinterpret_cast<uint32_t *>(p1)[(d + e) >> 1] = bf16_pair(x[u][0], x[u][1]);
-            reinterpret_cast<uint32_t *>(p2)[(d + e) >> 1] = bf16_pair(x[u][0] - h.x, x[u][1] - h.y);
+            reinterpret_cast<uint2 *>(p1)[d] = make_uint2(bf16_pair(x.x, x.y), bf16_pair(x.z, x.w));
+            reinterpret_cast<uint2 *>(p2)[d] = make_uint2(bf16_pair(x.x - h.x, x.y - h.y), bf16_pair(x.z - h.z, x.w - h.w));
           }
         }
       }
@@ -848,10 +888,14 @@ int flat_planes(b200_ctx *ctx, cudaStream_t stream, OperandView &v, PlaneKind ki
       b200::launch(ctx, pack_mix_flat_kernel, dim3(static_cast<unsigned>(need < cap ? need : cap)), dim3(256), 0, stream, 1u,
                    static_cast<const float4 *>(src), static_cast<float4 *>(p0), static_cast<uint2 *>(p1), static_cast<uint2 *>(p2), n4);
     } else {
-      // lanes of a warp per line: enough for its pairs, at most all
+      // threads of a CTA per line: enough for 16 bytes each, at most all; as many lines at once per thread as
+      // leave two CTAs to an SM
+      const uint32_t wide = kind == kPlanesHalf ? 8u : 4u;
       uint32_t shift = 0;
-      while (shift < 5u && (2u << shift) < key.pad) ++shift;
-      const unsigned long long need = ((key.lines << shift) + 255ull) / 256ull;
+      while (shift < 8u && (wide << shift) < key.line) ++shift;
+      const unsigned long long ctas = ((key.lines << shift) + 255ull) / 256ull, two = 2ull * ctx->sm_count;
+      unsigned long long need = (ctas + kPadUnits - 1u) / kPadUnits;
+      if (need < two) need = ctas < two ? ctas : two;
       const dim3 grid(static_cast<unsigned>(need < cap ? need : cap));
       if (kind == kPlanesHalf)
         b200::launch(ctx, pad_lines_kernel<kPlanesHalf, __half>, grid, dim3(256), 0, stream, 1u, static_cast<const __half *>(src), p0, p1, p2, key.line, key.pad, static_cast<unsigned long long>(key.lines), shift);
