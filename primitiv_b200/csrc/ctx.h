@@ -237,7 +237,7 @@ int gemm_skinny(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 int gemm_mma(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // fp32 modes, tcgen05 fed by the kernel's own loads: any shape, any alignment (gemm_direct.cu).
 int gemm_direct(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
-int gemm_direct_init(b200_ctx *ctx);   // fills cluster_room and cluster_room_two
+int gemm_find_rooms(b200_ctx *ctx);   // fills cluster_room and cluster_room_two
 // tcgen05 path.  tc_eligible() says whether the operands meet TMA's alignment rules.
 bool gemm_tc_eligible(const b200_ctx *ctx, const GemmArgs &g);
 int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);

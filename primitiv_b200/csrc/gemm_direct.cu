@@ -508,30 +508,6 @@ double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g) {
   return choose(ctx, g, wide_a(g) && wide_b(g)).us;
 }
 
-int gemm_direct_init(b200_ctx *ctx) {
-  auto kernel = gemm_direct_kernel<true, true, 64u, false>;
-  constexpr uint32_t kSmem = kDirectSmem<true, true, 64u>;
-  B200_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
-  for (unsigned s = 1; s <= 8u; ++s) {
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = s;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(s);
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    for (int two = 0; two < 2; ++two) {
-      int *room = two ? &ctx->cluster_room_two[s] : &ctx->cluster_room[s];
-      cfg.blockDim = dim3(two ? 128u : kFeedThreads + 32u);   // what the kernels of gemm_mma.cuh that share an SM have
-      cfg.dynamicSmemBytes = two ? 104u * 1024u : kSmem;
-      B200_CUDA_TRY(cudaOccupancyMaxActiveClusters(room, kernel, &cfg));
-      if (*room < 1) *room = 1;
-    }
-  }
-  return B200_OK;
-}
-
 int gemm_direct(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream) {
   if (g.mode != B200_MODE_FP32_3XTF32 && g.mode != B200_MODE_FP32_3XFP16) return B200_ERR_INVALID_ARG;
   DirectParams p;

@@ -77,18 +77,22 @@ MmaChoice choose(const b200_ctx *ctx, const GemmArgs &g, const MmaProblem &p) {
     const double tiles = static_cast<double>((p.a.mn + kTileM[t] - 1) / kTileM[t]) * ((p.b.mn + kTileN[t] - 1) / kTileN[t]) * g.groups;
     const int *clusters = t <= kTile64x64 ? ctx->cluster_room_two : ctx->cluster_room;
     for (uint32_t s = 1; s <= 8u && s <= p.kt; ++s) {
-      // (a cluster has to fit a GPC: 32 clusters of eight, two CTAs to an SM, do not run at once, nor does half of
-      // one more count; four 4096-wide layers of halves over 8 columns spent twice the time so)
-      double waves = tiles / clusters[s];
-      if (s > 1u) waves = static_cast<double>(static_cast<uint64_t>(waves + 0.999));
-      if (p.kind == kMmaFp32) waves = static_cast<double>(static_cast<uint64_t>(waves + 0.999));   // (bound by arithmetic: a last wave costs a whole one)
-      const double load = waves > 1.0 ? waves : 1.0;
+      // A cluster has to find its SMs free in one GPC.  Of clusters of eight with two CTAs to an SM 33 fit an
+      // idle GPU, but a layer of 4096 halves over 8 columns that needs 32 of them waits for what the kernel in
+      // front still holds: 14 us in a chain, 9 with seven.  Hence a tenth in reserve.
+      const double waves = tiles / (s > 1u ? 0.9 * clusters[s] : clusters[s]);
+      const double whole = static_cast<double>(static_cast<uint64_t>(waves + 0.999));
+      // (what is bound by arithmetic, or comes in clusters, pays for a started wave)
+      const double load = waves <= 1.0 ? 1.0 : (p.kind == kMmaFp32 || s > 1u) ? 0.5 * (waves + whole) : waves;
       const double us = load * (static_cast<double>((p.kt + s - 1) / s) * step + kEnds[p.kind][t]) + (s > 1u ? 1.8 : 0.0);
       if (us < best.us) best = {t, s, us};
     }
   }
   return best;
 }
+
+// Never launched: what the driver is asked about.
+__global__ void room_kernel() { pdl_enter(); }
 
 // Tensor map of an operand for tiles of `rows`: the box and swizzle that gemm_mma.cuh's Layout describes.
 bool make_map(const b200_ctx *ctx, const MmaOperand &o, uint32_t k, uint32_t groups, uint32_t red, int es, uint32_t rows,
@@ -111,6 +115,29 @@ bool make_map(const b200_ctx *ctx, const MmaOperand &o, uint32_t k, uint32_t gro
 }
 
 }  // namespace
+
+int gemm_find_rooms(b200_ctx *ctx) {
+  for (unsigned s = 1; s <= 8u; ++s) {
+    for (int two = 0; two < 2; ++two) {
+      const unsigned smem = (two ? 106u : 200u) * 1024u;   // two CTAs of the smaller tiles fit an SM, one of everything else
+      B200_CUDA_TRY(cudaFuncSetAttribute(room_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute attr{};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = s;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.gridDim = dim3(s);
+      cfg.blockDim = dim3(128);
+      cfg.dynamicSmemBytes = smem;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int *room = two ? &ctx->cluster_room_two[s] : &ctx->cluster_room[s];
+      B200_CUDA_TRY(cudaOccupancyMaxActiveClusters(room, room_kernel, &cfg));
+      if (*room < 1) *room = 1;
+    }
+  }
+  return B200_OK;
+}
 
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g) {
   // (half planes lose less than TF32 ones where the sum is that short, see gemm_direct_estimate)
