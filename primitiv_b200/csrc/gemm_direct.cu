@@ -476,7 +476,7 @@ DirectChoice choose(const b200_ctx *ctx, const GemmArgs &g, bool wide) {
   static const struct { uint32_t cols; double wide, narrow; } kTiles[] = {{64, 0.68, 0.8}, {96, 1.0, 1.1}, {32, 0.56, 0.7}};
   const uint64_t kb = static_cast<uint64_t>((g.k + kDirectK - 1) / kDirectK) * g.red;
   const uint32_t fixed = gemm_fixed_slices(ctx, g);
-  DirectChoice best{64, fixed ? fixed : 1u, 1e30};
+  DirectChoice best{64, fixed > 8u ? 8u : fixed ? fixed : 1u, 1e30};   // (more slices than a cluster has CTAs: not this kernel's)
   for (const auto &t : kTiles) {
     if (t.cols == 96u && g.trans_b) continue;   // (a line of 96 columns does not divide among the threads)
     const double tiles = static_cast<double>((g.m + kDirectM - 1) / kDirectM) * ((g.n + t.cols - 1) / t.cols) * g.groups;

@@ -1381,13 +1381,17 @@ bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g) {
   return direct_ok(a.ptr, a.ld, a.batch_stride, a.nbatch, eb) && direct_ok(b.ptr, b.ld, b.batch_stride, b.nbatch, eb);
 }
 
-// The fp32 mode sums a contraction of up to 1024 terms in one order, given by the sizes alone: the same bits whether
-// the operands come in planes or are split by the kernel, whatever the tile.  Activations pass or block a
-// gradient by their sign, and one value near zero that falls to the other side moves the weight gradient of an
-// 800-wide layer over 200 items by 0.25 %: a choice of kernel or tile should not do that.  The order is that of
-// 256-row, 256-column pair tiles with slices of four k-blocks or more for the pairs they leave idle.
+// The fp32 mode sums a contraction of up to 1024 terms, or of a large product, in one order, given by the sizes alone: the
+// same bits whether the operands come in planes or are split by the kernel, whatever the tile.  Activations pass or
+// block a gradient by their sign, and one value near zero that falls to the other side moves the weight gradient
+// of an 800-wide layer over 200 items by 0.25 %: a choice of kernel or tile should not do that (nor one of the
+// gradient's last bits, which are the next step's weights, over the 67 million activations of 65536 items).  The order
+// is that of 256-row, 256-column pair tiles with slices of four k-blocks or more for the pairs they leave idle.
+// From 2^32 multiply-adds up little faster was measured (1272 x 1652 x 2098: 75.8 us, 73.6 with any tile and
+// split); long contractions below that gain up to half (256 x 256 x 2048: 24.7 -> 11.8) and go as speed has it.
 uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g) {
-  if (g.mode != B200_MODE_FP32_3XTF32 || g.red != 1u || g.k > 1024u) return 0u;
+  if (g.mode != B200_MODE_FP32_3XTF32 || g.red != 1u) return 0u;
+  if (g.k > 1024u && static_cast<double>(g.m) * g.n * g.k * g.groups < 4294967296.0) return 0u;
   const uint32_t kb = (g.k + 31u) / 32u;
   const uint32_t bn = g.n > 128u ? 256u : g.n > 64u ? 128u : 64u, rows = bn >= 128u && g.m > kBM ? 2u * kBM : kBM;
   const uint64_t tiles = static_cast<uint64_t>((g.m + rows - 1) / rows) * ((g.n + bn - 1) / bn) * g.groups;
@@ -1395,6 +1399,7 @@ uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g) {
   if (ctx->split_policy == 1 || kb < 16u || tiles * 2u > units) return 1u;
   uint64_t want = units / tiles;
   if (want > kb / 4u) want = kb / 4u;
+  if (want > 64u) want = 64u;
   const uint32_t per = (kb + static_cast<uint32_t>(want) - 1u) / static_cast<uint32_t>(want);
   return (kb + per - 1u) / per;
 }
