@@ -210,7 +210,8 @@ B200_API int b200_matmul_fw_bw_host(b200_ctx *ctx, int mode,
  * force_path: 0 = choose; 1 = CUDA-core kernel; 2 = tensor-core kernel (error if ineligible);
  * 3 = the CUDA-core kernels for one tiny extent (m <= 16 or k <= 16) against large ones (error if
  * the shape and layout are not one of theirs); 4 = the mma.sync
- * kernel; 5 = the tcgen05 kernel that loads its operands itself (fp32 modes only). */
+ * kernel; 5 = the tcgen05 kernel that loads its operands itself (fp32 modes only); 6 = the CUDA-core
+ * kernel for a few thousand outputs (fp32 storage only). */
 B200_API int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b,
                        const void *A, const void *B, void *C,
                        uint32_t m, uint32_t n, uint32_t k,

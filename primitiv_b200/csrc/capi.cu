@@ -316,6 +316,7 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   if (force_path == 3) return b200::gemm_skinny_eligible(g) ? b200::gemm_skinny(ctx, g, s) : B200_ERR_INVALID_ARG;
   if (force_path == 4) return b200::gemm_mma(ctx, g, s);
   if (force_path == 5) return b200::gemm_direct(ctx, g, s);
+  if (force_path == 6) return b200::gemm_serial(ctx, g, s);
   if (ctx->path_policy == 2 && eligible) return b200::gemm_tc(ctx, g, s);
   if (ctx->path_policy == 1) return b200::gemm_simt(ctx, g, s);
   // One tiny extent against large ones is HBM-bound.  Where the tensor-core path would first have to pack
@@ -325,8 +326,12 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   if (b200::gemm_skinny_eligible(g) && !b200::gemm_tc_reads_in_place(ctx, g)) return b200::gemm_skinny(ctx, g, s);
   // Below two million multiply-adds a 128-row tcgen05 tile is mostly padding.  A contraction of a few terms
   // would not even fill a k-step of mma.sync (800 x 200 x 10: 3.4 us on the CUDA cores, 4.1 us there).
-  if (static_cast<double>(m) * n * k * groups * red < 2097152.0)
-    return static_cast<uint64_t>(k) * red <= 16u ? b200::gemm_simt(ctx, g, s) : b200::gemm_mma(ctx, g, s);
+  // The serial kernel has the CUDA cores' own bits, and up to some 800 terms is faster too (10 x 200 x 800: 8.0 us, 9.7 by
+  // mma.sync; 48 x 74 x 491 4.9 and 7.8; 200 x 8 x 1000 9.3 and 6.7).
+  if (static_cast<double>(m) * n * k * groups * red < 2097152.0) {
+    if (static_cast<uint64_t>(k) * red <= 16u) return b200::gemm_simt(ctx, g, s);
+    return b200::gemm_serial_estimate(ctx, g) <= 1.1 * b200::gemm_mma_estimate(ctx, g) ? b200::gemm_serial(ctx, g, s) : b200::gemm_mma(ctx, g, s);
+  }
   // Large products belong to tcgen05 fed by TMA, small fp32 ones to tcgen05 fed by the kernel's own loads, thin and
   // ragged ones to mma.sync: whichever is estimated to take least.
   const double tc = b200::gemm_tc_estimate(ctx, g), direct = b200::gemm_direct_estimate(ctx, g);

@@ -230,6 +230,8 @@ inline bool tiny_or_thin(const GemmArgs &g) {
 
 // CUDA-core path: any shape, any alignment.
 int gemm_simt(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
+// The same sums for a few thousand fp32 outputs (gemm_simt.cu).
+int gemm_serial(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // CUDA-core kernels for products with one tiny extent against large ones (gemm_skinny.cu).
 bool gemm_skinny_eligible(const GemmArgs &g);
 int gemm_skinny(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
@@ -248,6 +250,7 @@ bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g);
+double gemm_serial_estimate(const b200_ctx *ctx, const GemmArgs &g);
 // The number of slices that every tcgen05 kernel cuts this contraction into; 0: each kernel as it likes.
 uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g);
 // Checks (and re-arms) the guard bands of every pool block; see b200_pool_check_guards.

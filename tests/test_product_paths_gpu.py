@@ -22,12 +22,14 @@ def product(a, b, ta, tb, m, n, k):
     return (b @ a.T).reshape(-1)                     # n rows of m: column-major m x n
 
 
-@pytest.mark.parametrize("path", [2, 4, 5], ids=["tcgen05", "mma_sync", "tcgen05_self_fed"])
+@pytest.mark.parametrize("path", [2, 4, 5, 6], ids=["tcgen05", "mma_sync", "tcgen05_self_fed", "serial"])
 @pytest.mark.parametrize("mode", list(MODES))
 @pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
 def test_paths_at_their_edges(ctx, path, mode, layout):
     if path == 5 and mode in ("tf32", "fp16"):
         pytest.skip("the self-fed kernel is for the fp32 modes")
+    if path == 6 and mode == "fp16":
+        pytest.skip("the serial kernel is for fp32 storage")
     ta, tb = (int(c == "t") for c in layout)
     kind = torch.float16 if mode == "fp16" else torch.float32
     gen = torch.Generator(device="cuda")
@@ -119,3 +121,22 @@ def test_tiny_products_carry_infinities_and_nans_as_fp32_does(ctx, layout):
                 finite = torch.isfinite(fine)
                 assert torch.equal(got[~finite & ~torch.isnan(fine)], fine[~finite & ~torch.isnan(fine)])
                 assert ((got - fine)[finite].abs() <= 1e-5 * fine[finite].abs()).all()
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+def test_serial_products_have_the_cuda_core_kernels_bits(ctx, layout):
+    ta, tb = (int(c == "t") for c in layout)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(12)
+    for m, n, k, groups, red in ((10, 200, 800, 1, 1), (1, 1, 17, 1, 1), (8, 16, 128, 1, 1), (9, 17, 129, 3, 1), (33, 31, 127, 1, 5), (7, 300, 257, 2, 1)):
+        count = groups * red
+        a, b = (torch.randn(count * s, device="cuda", generator=gen) for s in (m * k, k * n))
+        c = torch.randn(groups * m * n, device="cuda", generator=gen)
+        got = []
+        for path in (1, 6):
+            out = c.clone()
+            ctx.gemm(MODES["3xtf32"], ta, tb, a.data_ptr(), b.data_ptr(), out.data_ptr(), m, n, k, groups, red, m * k if groups > 1 else 0,
+                     m * k if red > 1 else 0, k * n if groups > 1 else 0, k * n if red > 1 else 0, m * n, m % 2 == 0, path)
+            got.append(out)
+        assert ctx.status_poll() == 0
+        assert torch.equal(*got), (m, n, k, groups, red)
