@@ -134,8 +134,8 @@ struct Feed {
       const float4 x = raw[i], hi = make_float4(round(x.x), round(x.y), round(x.z), round(x.w));
       asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(base + to + i * kToStep), "f"(hi.x), "f"(hi.y), "f"(hi.z), "f"(hi.w) : "memory");
       if constexpr (kFull) {
-        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(base + kPlane + to + i * kToStep), "f"(round(x.x - hi.x)), "f"(round(x.y - hi.y)),
-                     "f"(round(x.z - hi.z)), "f"(round(x.w - hi.w)) : "memory");
+        asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(base + kPlane + to + i * kToStep), "f"(round_rest(x.x - hi.x)), "f"(round_rest(x.y - hi.y)),
+                     "f"(round_rest(x.z - hi.z)), "f"(round_rest(x.w - hi.w)) : "memory");
         continue;
       }
       sts64(base + kPlane + to8 + i * kTo8Step, bf16x2(x.x, x.y), bf16x2(x.z, x.w));
@@ -144,8 +144,15 @@ struct Feed {
   }
 
  private:
-  // Nearest TF32, ties away, as in pack.cu.  Inf passes through; a nan that loses its pattern leaves one in x - hi.
+  // Nearest TF32, ties away, as in pack.cu.  Inf passes through; a nan can become anything, but x - hi is then the one
+  // that arithmetic makes, 0x7fffffff: bf16 keeps it, and so does this rounding of the rest (the plain one would make
+  // it -0).
   static __device__ __forceinline__ float round(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+  static __device__ __forceinline__ float round_rest(float x) {
+    uint32_t v;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(v) : "f"(x));
+    return __uint_as_float(v);
+  }
   static __device__ __forceinline__ uint32_t bf16x2(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&v);

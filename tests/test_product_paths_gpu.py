@@ -140,3 +140,33 @@ def test_serial_products_have_the_cuda_core_kernels_bits(ctx, layout):
             got.append(out)
         assert ctx.status_poll() == 0
         assert torch.equal(*got), (m, n, k, groups, red)
+
+
+# nans: what the GPU's own arithmetic makes (0x7fffffff), its negative, ones that a carry or a cut would turn into an infinity
+NAN_BITS = (0x7fffffff, -1, 0x7f800001, -0x7fffff, 0x7fc00000)
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32", "3xfp16"])
+def test_no_nan_of_an_operand_is_lost(ctx, mode, layout):
+    """Whatever the bits of a nan, the whole row (column) of sums that it is a term of is nan, and nothing else is:
+    the split into two terms must keep it in one of them.  Sizes on either side of the tiny ones."""
+    ta, tb = (int(c == "t") for c in layout)
+    inf = torch.full((1,), float("inf"), device="cuda")
+    for m, n, k in ((48, 72, 96), (9, 300, 50), (200, 8, 1000), (256, 256, 320), (300, 96, 1100)):
+        for side in (0, 1):
+            a, b = torch.ones(m * k, device="cuda"), torch.full((k * n,), 0.5, device="cuda")
+            x, lines, by_k = ((a, m, ta), (b, n, not tb))[side]
+            at = lambda i, p: i * k + p if by_k else p * lines + i
+            for i, bits in enumerate(NAN_BITS):
+                x.view(torch.int32)[at(i, 7 * i + 3)] = bits
+            x[at(5, 0):at(5, 0) + 1] = inf - inf          # computed on the device
+            want = torch.zeros(n, m, dtype=torch.bool, device="cuda")
+            (want if side else want.T)[:6] = True
+            for path in (0, 4, 5, 6) if mode != "tf32" else (0, 4, 6):
+                if mode == "tf32" and n >= 16 and m * n * k >= 2097152:
+                    continue                               # (not split: 0x7f800001 cut to TF32 is an infinity)
+                c = torch.empty(m * n, device="cuda")
+                ctx.gemm(MODES[mode], ta, tb, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, 1, 1, 0, 0, 0, 0, 0, False, path)
+                assert ctx.status_poll() == 0
+                assert torch.equal(torch.isnan(c.view(n, m)), want), (m, n, k, side, path)
