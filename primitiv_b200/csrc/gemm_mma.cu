@@ -140,8 +140,9 @@ int gemm_find_rooms(b200_ctx *ctx) {
 }
 
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g) {
-  // (half planes lose less than TF32 ones where the sum is that short, see gemm_direct_estimate)
-  if (g.mode == B200_MODE_FP32_3XFP16 && static_cast<uint64_t>(g.k) * g.red < 64u && !tiny_or_thin(g)) return 1e30;
+  // (half planes lose less than TF32 ones where the sum is that short, see gemm_direct_estimate; this kernel takes
+  // what cannot have them)
+  if (g.mode == B200_MODE_FP32_3XFP16 && static_cast<uint64_t>(g.k) * g.red < 64u && !tiny_or_thin(g) && gemm_tc_eligible(ctx, g)) return 1e30;
   const MmaProblem p = describe(g);
   // (the fixed part was fitted with the rest: `ends` has it)
   return choose(ctx, g, p).us + 0.5;

@@ -170,3 +170,32 @@ def test_no_nan_of_an_operand_is_lost(ctx, mode, layout):
                 ctx.gemm(MODES[mode], ta, tb, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, 1, 1, 0, 0, 0, 0, 0, False, path)
                 assert ctx.status_poll() == 0
                 assert torch.equal(torch.isnan(c.view(n, m)), want), (m, n, k, side, path)
+
+
+# two batch axes: every matrix of the batch its own, and the sum over `red` of them
+TWO_AXES = [(256, 256, 20, 8, 3), (256, 256, 100, 4, 5), (515, 129, 333, 2, 3), (48, 40, 30, 3, 2), (128, 512, 700, 2, 2)]
+
+
+def two_axes_error(ctx, mode, layout, size, path):
+    """Relative error (norms) of such a product against 64 bits."""
+    ta, tb = (int(c == "t") for c in layout)
+    m, n, k, groups, red = size
+    kind = torch.float16 if mode == "fp16" else torch.float32
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(5)
+    a, b = (torch.rand(groups * red * s, device="cuda", generator=gen).sub_(0.5).to(kind) for s in (m * k, k * n))
+    c = torch.empty(groups * m * n, device="cuda", dtype=kind)
+    ctx.gemm(MODES[mode], ta, tb, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, groups, red, m * k * red, m * k,
+             k * n * red, k * n, m * n, False, path)
+    assert ctx.status_poll() == 0
+    a, b = a.double().view(groups * red, -1), b.double().view(groups * red, -1)
+    want = torch.cat([sum(product(a[g * red + r], b[g * red + r], ta, tb, m, n, k) for r in range(red)) for g in range(groups)])
+    return float((c.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+@pytest.mark.parametrize("mode", list(MODES))
+def test_two_batch_axes_are_taken_in_every_mode(ctx, mode, layout):
+    """No kernel of planes takes them, so the choice has to end at one that does, whatever the length of the sum."""
+    for size in TWO_AXES:
+        assert two_axes_error(ctx, mode, layout, size, 0) <= TOL[mode], size
