@@ -221,11 +221,13 @@ struct GemmArgs {
   int accumulate;
 };
 
-// Tiny and thin products are bound by latency or by the large operand's bytes: even in TF32 mode they are
-// given fp32 arithmetic, or as good a split (gemm_mma.cuh), which costs next to nothing there.
-inline bool tiny_or_thin(const GemmArgs &g) {
+// Products with fp32 arithmetic, or as good a split (gemm_mma.cuh), in every mode of fp32 storage, TF32 included: tiny and
+// thin ones, which are bound by latency or by the large operand's bytes, so that it costs next to nothing; and those that step
+// through an operand along both batch axes, which planes cannot follow.
+inline bool has_fp32_sums(const GemmArgs &g) {
   const double macs = static_cast<double>(g.m) * g.n * g.k * g.groups * g.red;
-  return macs < 2097152.0 || g.n < 16u || (g.m < 32u && macs < 67108864.0);
+  if (macs < 2097152.0 || g.n < 16u || (g.m < 32u && macs < 67108864.0)) return true;
+  return g.groups > 1u && g.red > 1u && ((g.a_gs != 0u && g.a_rs != 0u) || (g.b_gs != 0u && g.b_rs != 0u));
 }
 
 // CUDA-core path: any shape, any alignment.

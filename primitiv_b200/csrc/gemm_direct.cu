@@ -509,7 +509,7 @@ bool wide_b(const GemmArgs &g) { return all_wide(g.B, g.trans_b ? g.n : g.k, g.b
 double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g) {
   if (g.mode != B200_MODE_FP32_3XTF32 && g.mode != B200_MODE_FP32_3XFP16) return 1e30;
   if (ctx->correction_policy == 1) return 1e30;   // the caller wants TF32 planes throughout
-  if (tiny_or_thin(g)) return 1e30;
+  if (has_fp32_sums(g)) return 1e30;
   // (half planes lose less than this kernel where the sum is that short: 1.2e-7 against 1.6e-7 at 48 terms)
   if (g.mode == B200_MODE_FP32_3XFP16 && static_cast<uint64_t>(g.k) * g.red < 64u) return 1e30;
   return choose(ctx, g, wide_a(g) && wide_b(g)).us;

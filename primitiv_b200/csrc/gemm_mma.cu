@@ -32,7 +32,7 @@ struct MmaProblem {
 
 MmaProblem describe(const GemmArgs &g) {
   MmaProblem p;
-  p.kind = g.mode == B200_MODE_FP16 ? kMmaHalf : g.mode == B200_MODE_TF32 && !tiny_or_thin(g) ? kMmaTf32 : kMmaFp32;
+  p.kind = g.mode == B200_MODE_FP16 ? kMmaHalf : g.mode == B200_MODE_TF32 && !has_fp32_sums(g) ? kMmaTf32 : kMmaFp32;
   p.es = elem_bytes(g.mode);
   p.a = {g.A, g.m, g.trans_a != 0, g.trans_a ? g.k : g.m, g.a_gs, g.a_rs};
   p.b = {g.B, g.n, g.trans_b == 0, g.trans_b ? g.n : g.k, g.b_gs, g.b_rs};
@@ -141,8 +141,8 @@ int gemm_find_rooms(b200_ctx *ctx) {
 
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g) {
   // (half planes lose less than TF32 ones where the sum is that short, see gemm_direct_estimate; this kernel takes
-  // what cannot have them)
-  if (g.mode == B200_MODE_FP32_3XFP16 && static_cast<uint64_t>(g.k) * g.red < 64u && !tiny_or_thin(g) && gemm_tc_eligible(ctx, g)) return 1e30;
+  // what cannot have them, two batch axes among it)
+  if (g.mode == B200_MODE_FP32_3XFP16 && static_cast<uint64_t>(g.k) * g.red < 64u && !has_fp32_sums(g)) return 1e30;
   const MmaProblem p = describe(g);
   // (the fixed part was fitted with the rest: `ends` has it)
   return choose(ctx, g, p).us + 0.5;
@@ -177,7 +177,7 @@ int gemm_mma(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream) {
   }
   p.A = q.a.ptr; p.lda = q.a.ld; p.a_gs = q.a.gs; p.a_rs = q.a.rs;
   p.B = q.b.ptr; p.ldb = q.b.ld; p.b_gs = q.b.gs; p.b_rs = q.b.rs;
-  p.mend = q.kind == kMmaFp32 && tiny_or_thin(g) ? 1u : 0u;
+  p.mend = q.kind == kMmaFp32 && has_fp32_sums(g) ? 1u : 0u;
   p.tiles_m = (p.m + kTileM[c.tile] - 1) / kTileM[c.tile];
   p.tiles_n = (p.n + kTileN[c.tile] - 1) / kTileN[c.tile];
   p.kb = q.kb;

@@ -268,8 +268,8 @@ __device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-// An infinite operand makes x - hi a nan, or meets the zero it left of another one.  Tiny and thin products, which are the
-// CUDA cores' by their numerics, sum an element that is not finite again as those do.
+// An infinite operand makes x - hi a nan, or meets the zero it left of another one.  Products that are the CUDA
+// cores' by their numerics (has_fp32_sums) sum an element that is not finite again as those do.
 template <bool KA, bool KB>
 __device__ __noinline__ float plain_sum(const MmaParams &p, uint32_t g, uint32_t i, uint32_t j) {
   float v = 0.f;

@@ -1405,7 +1405,7 @@ uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g) {
 }
 
 double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g) {
-  if (!gemm_tc_eligible(ctx, g) || (g.mode != B200_MODE_FP16 && tiny_or_thin(g))) return 1e30;
+  if (!gemm_tc_eligible(ctx, g) || (g.mode != B200_MODE_FP16 && has_fp32_sums(g))) return 1e30;
   OperandView a, b;
   operand_views(g, &a, &b);
   const bool half = g.mode == B200_MODE_FP16 || g.mode == B200_MODE_FP32_3XFP16;

@@ -199,3 +199,22 @@ def test_two_batch_axes_are_taken_in_every_mode(ctx, mode, layout):
     """No kernel of planes takes them, so the choice has to end at one that does, whatever the length of the sum."""
     for size in TWO_AXES:
         assert two_axes_error(ctx, mode, layout, size, 0) <= TOL[mode], size
+
+
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32", "3xfp16"])
+def test_two_batch_axes_keep_fp32_sums(ctx, mode, layout):
+    """As precise as the CUDA cores (path 1), the single-pass mode included, and infinite where those are."""
+    for size in TWO_AXES:
+        assert two_axes_error(ctx, mode, layout, size, 0) <= 1.05 * two_axes_error(ctx, mode, layout, size, 1), size
+    ta, tb = (int(c == "t") for c in layout)
+    m, n, k, groups, red = 256, 256, 100, 2, 3
+    a, b = torch.ones(groups * red * m * k, device="cuda"), torch.full((groups * red * k * n,), 0.5, device="cuda")
+    at = (red + 1) * m * k                                # second matrix of the second group, element (0, 0)
+    a[at] = float("inf")
+    c = torch.empty(groups * m * n, device="cuda")
+    ctx.gemm(MODES[mode], ta, tb, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, groups, red, m * k * red, m * k, k * n * red, k * n, m * n)
+    assert ctx.status_poll() == 0
+    want = torch.full((groups, n, m), 0.5 * k * red, device="cuda")
+    want[1, :, 0] = float("inf")
+    assert torch.equal(c.view_as(want), want)
