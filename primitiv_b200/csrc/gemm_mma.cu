@@ -77,6 +77,7 @@ MmaChoice choose(const b200_ctx *ctx, const GemmArgs &g, const MmaProblem &p) {
     const double tiles = static_cast<double>((p.a.mn + kTileM[t] - 1) / kTileM[t]) * ((p.b.mn + kTileN[t] - 1) / kTileN[t]) * g.groups;
     const int *clusters = t <= kTile64x64 ? ctx->cluster_room_two : ctx->cluster_room;
     for (uint32_t s = 1; s <= 8u && s <= p.kt; ++s) {
+      if (t == kTile128x128 && p.kind == kMmaHalf && (p.kt + s - 1) / s > kMmaHalfRun) continue;   // (it has no second set of registers)
       // A cluster has to find its SMs free in one GPC.  Of clusters of eight with two CTAs to an SM 33 fit an
       // idle GPU, but a layer of 4096 halves over 8 columns that needs 32 of them waits for what the kernel in
       // front still holds: 14 us in a chain, 9 with seven.  Hence a tenth in reserve.

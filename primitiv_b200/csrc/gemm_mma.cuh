@@ -29,7 +29,8 @@
 //
 // The tensor core truncates when it adds into its accumulator (see gemm_tc.cu); the fp32 modes
 // therefore promote their accumulators to a second set of registers after every k-tile, and keep the small
-// terms out of them.
+// terms out of them.  Halves, which the CUDA cores summed without that bias, are promoted every kMmaHalfRun k-tiles: a
+// thousand terms lose 2e-6 of their sum, where the result is rounded to 2e-4 (a million terms in one run lost 7.5e-4 to 6e-3).
 #ifndef PRIMITIV_B200_CSRC_GEMM_MMA_CUH_
 #define PRIMITIV_B200_CSRC_GEMM_MMA_CUH_
 
@@ -301,12 +302,14 @@ struct MmaTile {
   static constexpr uint32_t kSmem = (STAGES * kStage > kOut ? STAGES * kStage : kOut) + 1024u;   // + alignment of the swizzles
 };
 
-// KA / KB: operand K-major (true) or MN-major.  LOAD: how operands are fetched.
-template <int KIND, int BM, int BN, int WM, int WN, int STAGES, bool KA, bool KB, int LOAD>
+// KA / KB: operand K-major (true) or MN-major.  LOAD: how operands are fetched.  RUNS (halves): sums longer than
+// kMmaHalfRun k-tiles; a kernel of its own, as the second set of registers costs a thin product of 640 terms 0.2 us.
+template <int KIND, int BM, int BN, int WM, int WN, int STAGES, bool KA, bool KB, int LOAD, bool RUNS>
 __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThreads) gemm_mma_kernel(const __grid_constant__ MmaParams p) {
   using Tile = MmaTile<KIND, BM, BN, WM, WN, STAGES>;
   using T = typename std::conditional<KIND == kMmaHalf, __half, float>::type;
   constexpr int kES = Tile::kES, NT = Tile::kThreads, MT = WM / 16, NB = WN / 8;
+  constexpr bool kSums = KIND == kMmaFp32 || RUNS;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES];
   __shared__ int s_abort;
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
   }
 
   float acc[MT][NB][4];
-  float sum[KIND == kMmaFp32 ? MT : 1][KIND == kMmaFp32 ? NB : 1][4], cor[KIND == kMmaFp32 ? MT : 1][KIND == kMmaFp32 ? NB : 1][4];
+  float sum[kSums ? MT : 1][kSums ? NB : 1][4], cor[KIND == kMmaFp32 ? MT : 1][KIND == kMmaFp32 ? NB : 1][4];
 #pragma unroll
   for (int i = 0; i < MT; ++i)
 #pragma unroll
@@ -341,7 +344,8 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         acc[i][j][q] = 0.f;
-        if constexpr (KIND == kMmaFp32) sum[i][j][q] = cor[i][j][q] = 0.f;
+        if constexpr (kSums) sum[i][j][q] = 0.f;
+        if constexpr (KIND == kMmaFp32) cor[i][j][q] = 0.f;
       }
 
   pdl_wait_previous();
@@ -450,6 +454,19 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
           }
         }
       }
+      if constexpr (RUNS) {
+        if ((it - (STAGES - 2u)) % kMmaHalfRun == 0u) {   // that many k-tiles are in
+#pragma unroll
+          for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int j = 0; j < NB; ++j)
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                sum[i][j][q] += acc[i][j][q];
+                acc[i][j][q] = 0.f;
+              }
+        }
+      }
     }
   }
   if constexpr (LOAD != kMmaTma) asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -468,6 +485,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
           const uint32_t mm = wm + i * 16u + gq + ((q >> 1) << 3), nn = wn + j * 8u + t * 2u + (q & 1);
           float v = acc[i][j][q];
           if constexpr (KIND == kMmaFp32) v = sum[i][j][q] + cor[i][j][q];
+          if constexpr (RUNS) v += sum[i][j][q];
           out[nn * Tile::kPitch + mm] = v;
         }
   }
@@ -552,10 +570,10 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
 }
 
 // Launches one instance.
-template <int KIND, int BM, int BN, int WM, int WN, int STAGES, bool KA, bool KB, int LOAD>
+template <int KIND, int BM, int BN, int WM, int WN, int STAGES, bool KA, bool KB, int LOAD, bool RUNS>
 int mma_launch(b200_ctx *ctx, const MmaParams &p, cudaStream_t stream) {
   using Tile = MmaTile<KIND, BM, BN, WM, WN, STAGES>;
-  auto kernel = gemm_mma_kernel<KIND, BM, BN, WM, WN, STAGES, KA, KB, LOAD>;
+  auto kernel = gemm_mma_kernel<KIND, BM, BN, WM, WN, STAGES, KA, KB, LOAD, RUNS>;
   if (Tile::kSmem > 48u * 1024u) {   // opt in once per device
     static std::atomic<unsigned long long> done{0};
     const unsigned long long bit = 1ull << (ctx->device & 63);
@@ -570,35 +588,43 @@ int mma_launch(b200_ctx *ctx, const MmaParams &p, cudaStream_t stream) {
   return static_cast<int>(cudaGetLastError());
 }
 
-template <int KIND, int BM, int BN, int WM, int WN, int STAGES, int LOAD>
+template <int KIND, int BM, int BN, int WM, int WN, int STAGES, int LOAD, bool RUNS>
 int mma_launch_layout(b200_ctx *ctx, const MmaParams &p, bool ka, bool kb, cudaStream_t stream) {
-  if (ka) return kb ? mma_launch<KIND, BM, BN, WM, WN, STAGES, true, true, LOAD>(ctx, p, stream)
-                    : mma_launch<KIND, BM, BN, WM, WN, STAGES, true, false, LOAD>(ctx, p, stream);
-  return kb ? mma_launch<KIND, BM, BN, WM, WN, STAGES, false, true, LOAD>(ctx, p, stream)
-            : mma_launch<KIND, BM, BN, WM, WN, STAGES, false, false, LOAD>(ctx, p, stream);
+  if (ka) return kb ? mma_launch<KIND, BM, BN, WM, WN, STAGES, true, true, LOAD, RUNS>(ctx, p, stream)
+                    : mma_launch<KIND, BM, BN, WM, WN, STAGES, true, false, LOAD, RUNS>(ctx, p, stream);
+  return kb ? mma_launch<KIND, BM, BN, WM, WN, STAGES, false, true, LOAD, RUNS>(ctx, p, stream)
+            : mma_launch<KIND, BM, BN, WM, WN, STAGES, false, false, LOAD, RUNS>(ctx, p, stream);
+}
+
+template <int KIND, int BM, int BN, int WM, int WN, int STAGES, bool RUNS>
+int mma_launch_load(b200_ctx *ctx, const MmaParams &p, bool ka, bool kb, cudaStream_t stream) {
+  if (p.load == kMmaTma) return mma_launch_layout<KIND, BM, BN, WM, WN, STAGES, kMmaTma, RUNS>(ctx, p, ka, kb, stream);
+  if constexpr (KIND == kMmaHalf) {
+    if (p.load == kMmaSingle) return mma_launch_layout<KIND, BM, BN, WM, WN, STAGES, kMmaSingle, RUNS>(ctx, p, ka, kb, stream);
+  }
+  return mma_launch_layout<KIND, BM, BN, WM, WN, STAGES, kMmaWord, RUNS>(ctx, p, ka, kb, stream);
 }
 
 template <int KIND, int BM, int BN, int WM, int WN, int STAGES>
-int mma_launch_load(b200_ctx *ctx, const MmaParams &p, bool ka, bool kb, cudaStream_t stream) {
-  if (p.load == kMmaTma) return mma_launch_layout<KIND, BM, BN, WM, WN, STAGES, kMmaTma>(ctx, p, ka, kb, stream);
+int mma_launch_runs(b200_ctx *ctx, const MmaParams &p, bool ka, bool kb, cudaStream_t stream) {
   if constexpr (KIND == kMmaHalf) {
-    if (p.load == kMmaSingle) return mma_launch_layout<KIND, BM, BN, WM, WN, STAGES, kMmaSingle>(ctx, p, ka, kb, stream);
+    if (p.kt_per > kMmaHalfRun) return mma_launch_load<KIND, BM, BN, WM, WN, STAGES, true>(ctx, p, ka, kb, stream);
   }
-  return mma_launch_layout<KIND, BM, BN, WM, WN, STAGES, kMmaWord>(ctx, p, ka, kb, stream);
+  return mma_launch_load<KIND, BM, BN, WM, WN, STAGES, false>(ctx, p, ka, kb, stream);
 }
 
 // The tiles of one kind.
 template <int KIND>
 int mma_launch_tile(b200_ctx *ctx, const MmaParams &p, int tile, bool ka, bool kb, cudaStream_t stream) {
   switch (tile) {
-    case kTile128x8: return mma_launch_load<KIND, 128, 8, 32, 8, 6>(ctx, p, ka, kb, stream);
-    case kTile128x16: return mma_launch_load<KIND, 128, 16, 32, 16, 5>(ctx, p, ka, kb, stream);
-    case kTile128x32: return mma_launch_load<KIND, 128, 32, 32, 32, 5>(ctx, p, ka, kb, stream);
-    case kTile64x64: return mma_launch_load<KIND, 64, 64, 32, 32, 4>(ctx, p, ka, kb, stream);
-    case kTile128x64: return mma_launch_load<KIND, 128, 64, 32, 32, 4>(ctx, p, ka, kb, stream);
+    case kTile128x8: return mma_launch_runs<KIND, 128, 8, 32, 8, 6>(ctx, p, ka, kb, stream);
+    case kTile128x16: return mma_launch_runs<KIND, 128, 16, 32, 16, 5>(ctx, p, ka, kb, stream);
+    case kTile128x32: return mma_launch_runs<KIND, 128, 32, 32, 32, 5>(ctx, p, ka, kb, stream);
+    case kTile64x64: return mma_launch_runs<KIND, 64, 64, 32, 32, 4>(ctx, p, ka, kb, stream);
+    case kTile128x64: return mma_launch_runs<KIND, 128, 64, 32, 32, 4>(ctx, p, ka, kb, stream);
     default:
-      // (the fp32 kinds' second set of accumulators does not leave the registers for it)
-      if constexpr (KIND != kMmaFp32) return mma_launch_load<KIND, 128, 128, 64, 32, 3>(ctx, p, ka, kb, stream);
+      // (a second set of accumulators does not leave the registers for it: not for the fp32 kinds, nor for runs)
+      if constexpr (KIND != kMmaFp32) return mma_launch_load<KIND, 128, 128, 64, 32, 3, false>(ctx, p, ka, kb, stream);
       else return B200_ERR_INVALID_ARG;
   }
 }

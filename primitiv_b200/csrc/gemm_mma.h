@@ -11,6 +11,7 @@ enum : int { kMmaHalf = 0, kMmaTf32 = 1, kMmaFp32 = 2 };   // storage and arithm
 // How a kernel fetches its operands: TMA (both meet its alignment rules), 4-byte copies, single halves.
 enum : int { kMmaTma = 16, kMmaWord = 4, kMmaSingle = 2 };
 enum : int { kTile128x8 = 0, kTile128x16, kTile128x32, kTile64x64, kTile128x64, kTile128x128 };
+constexpr uint32_t kMmaHalfRun = 16;   // k-tiles of 64 halves that the tensor core accumulates before their sum goes to registers
 
 struct alignas(64) MmaParams {
   CUtensorMap map_a, map_b;      // load == kMmaTma: dims {contiguous axis, other axis, matrix}

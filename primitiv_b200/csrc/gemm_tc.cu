@@ -53,7 +53,9 @@
 // while the tensor core works on the next chunk (two TMEM buffers).  The error
 // then no longer grows with the contraction length.  The single-pass modes use one
 // chunk per tile, and the two TMEM buffers overlap a tile's epilogue with the next
-// tile's main loop.
+// tile's main loop.  Except for halves that come here from the CUDA cores, whose sums have no such
+// bias: ragged lines and thin shapes are cut into chunks of 1024 terms (a million terms in one
+// chunk were off by 6e-3; half's own rounding is 2e-4).
 //
 // Every device-side wait is bounded (a few seconds, counted in SM clock cycles).  A wait that runs
 // out raises a CTA-wide abort flag, writes B200_ERR_KERNEL_TIMEOUT into the
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
   constexpr bool kF16 = kKind == 2 || kKind == 3;
   constexpr bool kMix = kKind == 4;
   constexpr bool kTable = kMix || kWide;   // the TMA boxes of a stage come from the host-built table
-  static_assert(!kChunked || kPasses == 3, "only the three-pass products are chunked");
+  static_assert(!kChunked || kPasses == 3 || kKind == 2, "only the three-pass products and halves are chunked");
   static_assert(!kWide || (kCtas == 2 && kKind == 2 && !kChunked), "the wide tile is a pair form for half storage");
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kMaxStages];
@@ -614,7 +616,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                   if (col0 + i < p.n) acc[j][i] *= row_scale * inv_scale_for(col_scale[col0 + i]);
               }
               // the three-pass kinds always store fp32 (half storage is the single-pass fp16 kind)
-              store_cols<8>(static_cast<float *>(p.C), base, p.m, p.n, col0, acc[j], p.accumulate != 0u);
+              if (kKind == 2 && p.out_half) store_cols<8>(static_cast<__half *>(p.C), base, p.m, p.n, col0, acc[j], p.accumulate != 0u);
+              else store_cols<8>(static_cast<float *>(p.C), base, p.m, p.n, col0, acc[j], p.accumulate != 0u);
             }
           }
         }
@@ -882,7 +885,9 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   // earns 5 % in its main loop: measured on 8192 x 8192 x 65536 halves, +4 % at k = 65536, -2.5 % at
   // k = 8192, break-even near 12 K.  pair_policy 2 = never, 3 = whenever n allows (tests).
   bool wide = false;
-  if (half_store && ctas == 2u && !fixed_scratch && g.n >= 512u && ctx->pair_policy != 2) {
+  // halves whose sums the CUDA cores would have: these keep their precision whatever the length
+  const bool long_halves = half_store && (has_fp32_sums(g) || !gemm_tc_reads_in_place(ctx, g));
+  if (half_store && ctas == 2u && !fixed_scratch && g.n >= 512u && ctx->pair_policy != 2 && !long_halves) {
     const uint64_t wide_tiles = static_cast<uint64_t>(p.tiles_m) * ((g.n + 511u) / 512u) * g.groups;
     const uint64_t k_total = static_cast<uint64_t>(g.k) * g.red;
     wide = ctx->pair_policy == 3 ||
@@ -1220,8 +1225,8 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   // (a longer chunk truncates more: products of one wave, whose slices are cut as speed has it, take chunks of half
   // the length and are no less precise for it, however long a slice is)
   const bool one_wave = may_split && launch_tiles <= static_cast<uint64_t>(ctx->sm_count) / ctas;
-  const uint32_t chunk_len = one_wave && !gemm_fixed_slices(ctx, g) ? kChunkKBlocks / 2u : kChunkKBlocks;
-  const bool chunked = passes == 3 && static_cast<uint64_t>(g.red) * p.kblocks > chunk_len;
+  const uint32_t chunk_len = one_wave && passes == 3 && !gemm_fixed_slices(ctx, g) ? kChunkKBlocks / 2u : kChunkKBlocks;
+  const bool chunked = (passes == 3 || long_halves) && static_cast<uint64_t>(g.red) * p.kblocks > chunk_len;
   p.chunk_kblocks = chunked ? chunk_len : g.red * p.kblocks;
   p.accumulate = g.accumulate ? 1u : 0u;
   p.out_half = half_store ? 1u : 0u;
@@ -1298,6 +1303,8 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
     allow(gemm_tc_kernel<false, 1, 4>);
     allow(gemm_tc_kernel<true, 2, 4>);
     allow(gemm_tc_kernel<false, 2, 4>);
+    allow(gemm_tc_kernel<true, 1, 2>);
+    allow(gemm_tc_kernel<true, 2, 2>);
     allow(gemm_tc_kernel<false, 2, 2, true>);
     if (e != cudaSuccess) rc = static_cast<int>(e);
     ctx->tc_smem_configured = (e == cudaSuccess);
@@ -1314,6 +1321,7 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
       else if (mix) b200::launch(ctx, gemm_tc_kernel<false, 2, 4>, gd, bd, smem_bytes, stream, 2u, p);
       else if (split16 && chunked) b200::launch(ctx, gemm_tc_kernel<true, 2, 3>, gd, bd, smem_bytes, stream, 2u, p);
       else if (split16) b200::launch(ctx, gemm_tc_kernel<false, 2, 3>, gd, bd, smem_bytes, stream, 2u, p);
+      else if (half_store && chunked) b200::launch(ctx, gemm_tc_kernel<true, 2, 2>, gd, bd, smem_bytes, stream, 2u, p);
       else if (chunked) b200::launch(ctx, gemm_tc_kernel<true, 2, 0>, gd, bd, smem_bytes, stream, 2u, p);
       else if (passes == 3) b200::launch(ctx, gemm_tc_kernel<false, 2, 0>, gd, bd, smem_bytes, stream, 2u, p);
       else if (!f16) b200::launch(ctx, gemm_tc_kernel<false, 2, 1>, gd, bd, smem_bytes, stream, 2u, p);
@@ -1327,6 +1335,8 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
       b200::launch(ctx, gemm_tc_kernel<true, 1, 3>, dim3(grid), dim3(kThreads), smem_bytes, stream, 1u, p);
     } else if (split16) {
       b200::launch(ctx, gemm_tc_kernel<false, 1, 3>, dim3(grid), dim3(kThreads), smem_bytes, stream, 1u, p);
+    } else if (half_store && chunked) {
+      b200::launch(ctx, gemm_tc_kernel<true, 1, 2>, dim3(grid), dim3(kThreads), smem_bytes, stream, 1u, p);
     } else if (chunked) {
       b200::launch(ctx, gemm_tc_kernel<true, 1, 0>, dim3(grid), dim3(kThreads), smem_bytes, stream, 1u, p);
     } else if (passes == 3) {

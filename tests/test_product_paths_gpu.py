@@ -218,3 +218,23 @@ def test_two_batch_axes_keep_fp32_sums(ctx, mode, layout):
     want = torch.full((groups, n, m), 0.5 * k * red, device="cuda")
     want[1, :, 0] = float("inf")
     assert torch.equal(c.view_as(want), want)
+
+
+# a sum of a million halves by steps, in one slice and in many; every form that the CUDA cores had
+@pytest.mark.parametrize("path", [0, 2, 4])
+@pytest.mark.parametrize("m,n,k,red", [(40, 24, 61, 16384), (40, 24, 1000003, 1), (200, 8, 500000, 1), (130, 200, 61, 8192), (136, 264, 999, 1024)])
+def test_long_half_sums_have_no_bias(ctx, path, m, n, k, red):
+    """Sums of positive halves that TMA cannot address, or of thin products, are as good as fp32 sums rounded to half
+    once.  Each result is then off by at most 2^-11 of itself; the mean of these errors, one per output, is zero
+    but for 2^-11 / sqrt(3 outputs), and fp32 sums add some 1e-5: their own truncation and promotion."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(9)
+    a, b = (torch.rand(red * s, device="cuda", generator=gen).mul_(2.0 ** -7).half() for s in (m * k, k * n))
+    c = torch.empty(m * n, device="cuda", dtype=torch.half)
+    ctx.gemm(MODES["fp16"], 0, 0, a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, 1, red, 0, m * k, 0, k * n, 0, False, path)
+    assert ctx.status_poll() == 0
+    a, b = a.view(red, k, m), b.view(red, n, k)
+    want = sum(torch.einsum("rkm,rnk->nm", a[i:i + 64].double(), b[i:i + 64].double()) for i in range(0, red, 64))
+    off = (c.view(n, m).double() / want - 1).flatten()
+    assert off.mean().abs() <= 4 * 2.0 ** -11 / (3 * m * n) ** 0.5 + 1e-5
+    assert off.abs().max() <= 2.0 ** -11 + 3e-5
