@@ -146,12 +146,11 @@ struct Feed {
  private:
   // Nearest TF32, ties away, as in pack.cu.  Inf passes through; a nan can become anything, but x - hi is then the one
   // that arithmetic makes, 0x7fffffff: bf16 keeps it, and so does this rounding of the rest (the plain one would make
-  // it -0).
+  // it -0; see gemm_mma.cuh).
   static __device__ __forceinline__ float round(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
   static __device__ __forceinline__ float round_rest(float x) {
-    uint32_t v;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(v) : "f"(x));
-    return __uint_as_float(v);
+    const int u = __float_as_int(x);
+    return __uint_as_float(static_cast<uint32_t>(__viaddmax_s32(u, 0x1000, u)) & 0xffffe000u);
   }
   static __device__ __forceinline__ uint32_t bf16x2(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);

@@ -221,21 +221,26 @@ __device__ __forceinline__ void frag_b(uint32_t (&b)[NB][2], uint32_t base, uint
 // x rounded to TF32, nearest with ties away, as in pack.cu.  Inf passes through (the carry stays inside
 // the mantissa); a nan can become anything here, -0 and inf among it.
 __device__ __forceinline__ uint32_t round_tf32(uint32_t u) { return (u + 0x1000u) & 0xffffe000u; }
-// The same rounding of every number, and a nan stays one.
 // The single-pass mode rounds its operands (the tensor core would cut them off, at three times the error).
 __device__ __forceinline__ uint32_t nearest_tf32(uint32_t u) {
   uint32_t v;
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(v) : "f"(__uint_as_float(u)));
   return v;
 }
-// The fp32 modes' fragments: x = hi + lo, both TF32.  Where x is a nan, x - hi is the one that arithmetic makes,
-// 0x7fffffff, which only the second rounding carries on (the first would make it -0).
+// The same for x - hi.  Where x is a nan that is the nan which arithmetic makes, 0x7fffffff: the carry would take it to
+// -0, so the larger of both integers stays, which for every other value is the sum (the intrinsic's addition wraps, and
+// it is one instruction: a 2088-wide TF32 layer over two items 10.4 us, by cvt.rna.tf32, which keeps nans too, 11.7).
+__device__ __forceinline__ uint32_t round_rest(float x) {
+  const int u = __float_as_int(x);
+  return static_cast<uint32_t>(__viaddmax_s32(u, 0x1000, u)) & 0xffffe000u;
+}
+// The fp32 modes' fragments: x = hi + lo, both TF32.
 template <int N>
 __device__ __forceinline__ void split_fp32(uint32_t (&x)[N], uint32_t (&lo)[N]) {
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     const uint32_t hi = round_tf32(x[i]);
-    lo[i] = nearest_tf32(__float_as_uint(__uint_as_float(x[i]) - __uint_as_float(hi)));
+    lo[i] = round_rest(__uint_as_float(x[i]) - __uint_as_float(hi));
     x[i] = hi;
   }
 }
