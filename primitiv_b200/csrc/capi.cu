@@ -334,13 +334,17 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   }
   // Large products belong to tcgen05 fed by TMA, small fp32 ones to tcgen05 fed by the kernel's own loads, thin and
   // ragged ones to mma.sync: whichever is estimated to take least.
-  const double tc = b200::gemm_tc_estimate(ctx, g), direct = b200::gemm_direct_estimate(ctx, g);
-  double mma = b200::gemm_mma_estimate(ctx, g);
+  const bool one_order = b200::gemm_fixed_slices(ctx, g) != 0u;
+  double tc = b200::gemm_tc_estimate(ctx, g, false), mma = b200::gemm_mma_estimate(ctx, g);
+  const double direct = b200::gemm_direct_estimate(ctx, g);
   // (unless mma.sync is clearly faster the kernels that share one order of summation have the product: 300 x 500 x 333
   // at 12.3 us against 10.6 was within the estimates' error)
-  if (b200::gemm_fixed_slices(ctx, g)) mma *= 1.3;
-  if (direct < tc && direct < mma) return b200::gemm_direct(ctx, g, s);
-  return mma < tc ? b200::gemm_mma(ctx, g, s) : b200::gemm_tc(ctx, g, s);
+  if (one_order) mma *= 1.3;
+  if (mma < tc && mma < direct) return b200::gemm_mma(ctx, g, s);
+  // Planes that happen to be held may only decide where both kernels give the same bits: the same call on the same operands
+  // has to give the same twice.
+  if (one_order) tc = b200::gemm_tc_estimate(ctx, g, true);
+  return direct < tc ? b200::gemm_direct(ctx, g, s) : b200::gemm_tc(ctx, g, s);
 }
 
 int b200_gemm_3xtf32_noalloc(b200_ctx *ctx, int trans_a, int trans_b, const void *A, const void *B,

@@ -249,7 +249,7 @@ int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g);
 // Microseconds either path would take on an otherwise idle GPU, the launch included: for choosing
 // between them.  1e30: not eligible.
-double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g);
+double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g, bool look);   // look: at the planes that are cached
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_serial_estimate(const b200_ctx *ctx, const GemmArgs &g);

@@ -823,9 +823,10 @@ TileCost tile_cost(int mode, bool mix) {
   return {passes == 3u ? 256u : 128u, mix ? 8u : 4u * passes, f16 ? 110e3 : 90e3};
 }
 
-// What fetching one operand costs before the product: nothing where TMA reads it in place or its planes are
-// cached; else a launch and the bytes it moves, at the rates of the kernels in pack.cu.
-double pack_us(const b200_ctx *ctx, const OperandView &v, int mode, bool is_b, uint32_t m) {
+// What fetching one operand costs before the product: nothing where TMA reads it in place; else a launch and the bytes it
+// moves, at the rates of the kernels in pack.cu.  Planes of the fp32 mode are taken to serve two products of a step, or, with
+// `look`, it is seen whether they are cached.  Those of the single-pass modes are of the same call.
+double pack_us(const b200_ctx *ctx, const OperandView &v, int mode, bool is_b, uint32_t m, bool look) {
   const double elems = static_cast<double>(v.mn) * v.k * (v.nbatch ? v.nbatch : 1u);
   if (mode == B200_MODE_FP16 || mode == B200_MODE_TF32) {
     if (direct_ok(v.ptr, v.ld, v.batch_stride, v.nbatch, elem_bytes(mode))) return 0.0;
@@ -834,9 +835,8 @@ double pack_us(const b200_ctx *ctx, const OperandView &v, int mode, bool is_b, u
   }
   if (mode == B200_MODE_FP32_3XFP16) return (v.mn_major ? 6.0 : 2.5) + elems * 8.0 / 4e6;
   if (is_b && v.mn_major && m > 1536u) return 2.0 + elems * 12.0 / 4e6;   // transposed
-  if (flat_cached(ctx, v, kPlanesMix)) return 0.0;
-  // (with the cache on, planes serve two products of a step)
-  return (ctx->planes.cap ? 0.6 : 1.0) * (2.0 + elems * 12.0 / 5e6);
+  if (look && flat_cached(ctx, v, kPlanesMix)) return 0.0;
+  return 0.6 * (2.0 + elems * 12.0 / 5e6);
 }
 
 // Shared body of gemm_tc and of the allocation-free entry point.  With
@@ -1414,7 +1414,7 @@ uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g) {
   return (kb + per - 1u) / per;
 }
 
-double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g) {
+double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g, bool look) {
   if (!gemm_tc_eligible(ctx, g) || (g.mode != B200_MODE_FP16 && has_fp32_sums(g))) return 1e30;
   OperandView a, b;
   operand_views(g, &a, &b);
@@ -1423,7 +1423,7 @@ double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g) {
   const bool mix = g.mode == B200_MODE_FP32_3XTF32 && ctx->correction_policy != 1;
   const uint32_t bk = half ? 64u : 32u;
   const TileChoice t = choose_tile(ctx, g, tile_cost(g.mode, mix), (g.k + bk - 1) / bk, one ? 2u : 1u, ctx->split_policy != 1);
-  return 3.0 + t.us + pack_us(ctx, a, g.mode, false, g.m) + pack_us(ctx, b, g.mode, true, g.m);
+  return 3.0 + t.us + pack_us(ctx, a, g.mode, false, g.m, look) + pack_us(ctx, b, g.mode, true, g.m, look);
 }
 
 int gemm_tc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream) {

@@ -238,3 +238,35 @@ def test_long_half_sums_have_no_bias(ctx, path, m, n, k, red):
     off = (c.view(n, m).double() / want - 1).flatten()
     assert off.mean().abs() <= 4 * 2.0 ** -11 / (3 * m * n) ** 0.5 + 1e-5
     assert off.abs().max() <= 2.0 ** -11 + 3e-5
+
+
+@pytest.mark.parametrize("mode", ["3xtf32", "tf32", "fp16"])
+def test_bits_do_not_depend_on_the_plane_cache(ctx, mode):
+    """Forward and backward with no planes held, with all that the plane kernels would keep, and with the cache off:
+    the same bits.  Sums of more than 1024 terms below 2^32 multiply-adds, whose order the kernels choose themselves."""
+    kind = torch.float16 if mode == "fp16" else torch.float32
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(2)
+    try:
+        for di, dj, dk, n in ((1024, 1536, 512, 1), (256, 2048, 256, 1), (515, 1100, 387, 2), (256, 1300, 1024, 3), (2048, 1111, 333, 1), (700, 1600, 900, 1)):
+            a, b, gy = (torch.randn(n * s, device="cuda", generator=gen).to(kind) for s in (di * dj, dj * dk, di * dk))
+            y, ga, gb = torch.empty_like(gy), torch.empty_like(a), torch.empty_like(b)
+
+            def step():
+                ctx.matmul_fw(MODES[mode], a.data_ptr(), b.data_ptr(), y.data_ptr(), di, dj, dk, n, n)
+                ctx.matmul_bw_ex(MODES[mode], a.data_ptr(), b.data_ptr(), gy.data_ptr(), ga.data_ptr(), gb.data_ptr(), di, dj, dk, n, n, False, False)
+                return [x.clone() for x in (y, ga, gb)]
+
+            ctx.operand_cache_enable(0)
+            off = step()
+            ctx.operand_cache_enable(1 << 30)
+            cold = step()
+            ctx.set_path_policy(2)      # every product by planes: they are all held afterwards
+            step()
+            ctx.set_path_policy(0)
+            held = step()
+            for x, others in zip(off, zip(cold, held)):
+                assert all(torch.equal(x, o) for o in others), (di, dj, dk, n)
+    finally:
+        ctx.set_path_policy(0)
+        ctx.operand_cache_enable(0)
