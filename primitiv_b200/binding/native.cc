@@ -8,7 +8,7 @@
 // elementwise operation of 64 elements, back to back: 5.3 us per call through ctypes, 2.7 us here.
 //
 // An argument that is neither a number nor None (a ctypes array or reference) is left to the ctypes
-// path: the wrappers report it and `op` hands the call to the fallback it was created with.
+// path: the wrappers report it and the call goes to the fallback it was created with.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -102,30 +102,55 @@ const Named kEntries[] = {
 
 PyObject *g_by_name = nullptr;    // name -> capsule-free integer: index into kEntries
 
-// ---- Caller: op(name, *args) of one context ---------------------------------------------------
+// ---- Caller: op(name, *args) ----
+//
+// It comes in two forms.  Over a fixed address it is a function of one context, whose owner outlives it.  Without one it is a
+// method, to be an attribute of a class: it is called with the object first and takes the context's address from
+// that object's `_address`, an integer, at each call.  The object is then kept alive by whoever holds the bound
+// method, a closed one has a 0 there, and a subclass can put its own method in place, as with a function
+// written in Python.
 
 struct Caller {
   PyObject_HEAD
   vectorcallfunc vectorcall;
-  b200_ctx *ctx;
-  PyObject *fallback;   // called with (name, *args) for what the wrappers do not take
+  bool method;
+  b200_ctx *ctx;        // unless it is a method
+  PyObject *fallback;   // called with the same arguments for what the wrappers do not take
   PyObject *fail;       // called with (code, name); raises
 };
 
+PyObject *g_address = nullptr;   // "_address"
+
+// The context of the object that a method is called on.  False, with no error set: it has no such integer.
+bool context_of(PyObject *object, b200_ctx **ctx) {
+  PyObject *address = PyObject_GetAttr(object, g_address);
+  const bool ok = address && PyLong_Check(address);
+  if (ok) *ctx = static_cast<b200_ctx *>(PyLong_AsVoidPtr(address));
+  Py_XDECREF(address);
+  if (!PyErr_Occurred()) return ok;
+  PyErr_Clear();
+  return false;
+}
+
 PyObject *caller_call(PyObject *self, PyObject *const *args, size_t nargsf, PyObject *kwnames) {
   Caller *c = reinterpret_cast<Caller *>(self);
-  const Py_ssize_t n = PyVectorcall_NARGS(nargsf);
-  if (n >= 1 && !kwnames && PyUnicode_CheckExact(args[0])) {
-    PyObject *at = PyDict_GetItemWithError(g_by_name, args[0]);   // borrowed
+  const Py_ssize_t n = PyVectorcall_NARGS(nargsf), skip = c->method ? 1 : 0;
+  if (n > skip && !kwnames && PyUnicode_CheckExact(args[skip])) {
+    PyObject *at = PyDict_GetItemWithError(g_by_name, args[skip]);   // borrowed
     if (!at && PyErr_Occurred()) return nullptr;
-    if (at) {
-      const long code = kEntries[PyLong_AsLong(at)].fn(c->ctx, args + 1, n - 1);
+    b200_ctx *ctx = c->ctx;
+    if (at && (!c->method || context_of(args[0], &ctx))) {
+      const long code = kEntries[PyLong_AsLong(at)].fn(ctx, args + skip + 1, n - skip - 1);
       if (code == 0) Py_RETURN_NONE;
-      if (code > 0) return PyObject_CallFunction(c->fail, "lO", code, args[0]);
+      if (code > 0) return PyObject_CallFunction(c->fail, "lO", code, args[skip]);
       if (PyErr_Occurred()) return nullptr;
     }
   }
   return PyObject_Vectorcall(c->fallback, args, nargsf, kwnames);
+}
+
+PyObject *caller_get(PyObject *self, PyObject *object, PyObject *) {
+  return object ? PyMethod_New(self, object) : Py_NewRef(self);
 }
 
 int caller_traverse(PyObject *self, visitproc visit, void *arg) {
@@ -134,23 +159,33 @@ int caller_traverse(PyObject *self, visitproc visit, void *arg) {
   return 0;
 }
 
-void caller_dealloc(PyObject *self) {
-  PyObject_GC_UnTrack(self);
+int caller_clear(PyObject *self) {
   Py_CLEAR(reinterpret_cast<Caller *>(self)->fallback);
   Py_CLEAR(reinterpret_cast<Caller *>(self)->fail);
+  return 0;
+}
+
+void caller_dealloc(PyObject *self) {
+  PyObject_GC_UnTrack(self);
+  caller_clear(self);
   PyObject_GC_Del(self);
 }
 
 PyTypeObject caller_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
 PyObject *make_caller(PyObject *, PyObject *args) {
-  unsigned long long ctx = 0;
-  PyObject *fallback, *fail;
-  if (!PyArg_ParseTuple(args, "KOO", &ctx, &fallback, &fail)) return nullptr;
+  PyObject *address, *fallback, *fail;
+  if (!PyArg_ParseTuple(args, "OOO", &address, &fallback, &fail)) return nullptr;
+  std::uintptr_t ctx = 0;
+  if (address != Py_None) {
+    ctx = reinterpret_cast<std::uintptr_t>(PyLong_AsVoidPtr(address));
+    if (!ctx && PyErr_Occurred()) return nullptr;
+  }
   Caller *c = PyObject_GC_New(Caller, &caller_type);
   if (!c) return nullptr;
   c->vectorcall = caller_call;
-  c->ctx = reinterpret_cast<b200_ctx *>(static_cast<std::uintptr_t>(ctx));
+  c->method = address == Py_None;
+  c->ctx = reinterpret_cast<b200_ctx *>(ctx);
   c->fallback = Py_NewRef(fallback);
   c->fail = Py_NewRef(fail);
   PyObject_GC_Track(reinterpret_cast<PyObject *>(c));
@@ -158,7 +193,8 @@ PyObject *make_caller(PyObject *, PyObject *args) {
 }
 
 PyMethodDef methods[] = {
-    {"caller", make_caller, METH_VARARGS, "caller(context, fallback, fail): op(name, *args) of one context"},
+    {"caller", make_caller, METH_VARARGS,
+     "caller(context, fallback, fail): op(name, *args) of the context at that address, or with None a method of objects with an `_address`"},
     {nullptr, nullptr, 0, nullptr},
 };
 
@@ -170,14 +206,17 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Fast calls into libprim
 PyMODINIT_FUNC PyInit__native() {
   caller_type.tp_name = "primitiv_b200._native.Caller";
   caller_type.tp_basicsize = sizeof(Caller);
-  caller_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC | Py_TPFLAGS_HAVE_VECTORCALL;
+  caller_type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_HAVE_GC | Py_TPFLAGS_HAVE_VECTORCALL | Py_TPFLAGS_METHOD_DESCRIPTOR;
   caller_type.tp_vectorcall_offset = offsetof(Caller, vectorcall);
   caller_type.tp_call = PyVectorcall_Call;
+  caller_type.tp_descr_get = caller_get;
   caller_type.tp_traverse = caller_traverse;
+  caller_type.tp_clear = caller_clear;
   caller_type.tp_dealloc = caller_dealloc;
   if (PyType_Ready(&caller_type) < 0) return nullptr;
   g_by_name = PyDict_New();
-  if (!g_by_name) return nullptr;
+  g_address = PyUnicode_InternFromString("_address");
+  if (!g_by_name || !g_address) return nullptr;
   for (long i = 0; i < static_cast<long>(sizeof(kEntries) / sizeof(kEntries[0])); ++i) {
     PyObject *at = PyLong_FromLong(i);
     if (!at || PyDict_SetItemString(g_by_name, kEntries[i].name, at) < 0) return nullptr;

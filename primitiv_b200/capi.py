@@ -5,11 +5,10 @@ Device memory and streams come from the caller (raw integer addresses, e.g.
 no compute of its own.
 
 ``lib()`` is the library through ctypes.  The entry points that a training step calls
-thousands of times go through ``_native.so`` (binding/native.cc) instead, which takes plain
+thousands of times go through ``_native`` (binding/native.cc) instead, which takes plain
 numbers and None only; ``Context.op`` tries it first.
 """
 import ctypes
-import functools
 import os
 
 MODE_FP32_3XTF32 = 0
@@ -131,6 +130,11 @@ def lib():
             fn = getattr(handle, name)
             fn.restype = res
             fn.argtypes = args
+        try:
+            from . import _native
+        except ImportError as e:
+            raise ImportError("primitiv_b200/_native.so is not built (run `python -m primitiv_b200.build`): %s" % e) from e
+        Context.op = _native.caller(None, Context.op, _check)
         _LIB = handle
     return _LIB
 
@@ -140,34 +144,21 @@ def _check(code, what=""):
         raise B200Error(code, what)
 
 
-def _call_ctypes(handle, name, *args):
-    _check(getattr(lib(), name)(handle, *args), name)
-
-
-def _caller(handle):
-    """``op`` of one context: the native wrapper where there is one and the arguments are plain."""
-    lib()
-    try:
-        from . import _native
-    except ImportError as e:
-        raise ImportError("primitiv_b200/_native.so is not built (run `python -m primitiv_b200.build`): %s" % e) from e
-    return _native.caller(handle.value, functools.partial(_call_ctypes, handle), _check)
-
-
 class Context:
     """One b200_ctx (one GPU).  Mirrors the lifetime of a primitiv::devices::B200 object."""
+
+    _address = 0   # of the b200_ctx while it is open: `op` reads it at each call
 
     def __init__(self, device_id=0):
         self._h = _vp()
         _check(lib().b200_ctx_create(device_id, ctypes.byref(self._h)), "b200_ctx_create")
+        self._address = self._h.value
         self.device_id = device_id
-        self.op = _caller(self._h)
 
     def close(self):
         if self._h:
-            del self.op   # it holds the context's address
-            lib().b200_ctx_destroy(self._h)
-            self._h = _vp()
+            h, self._h, self._address = self._h, _vp(), 0
+            lib().b200_ctx_destroy(h)
 
     def __del__(self):
         try:
@@ -299,9 +290,9 @@ class Context:
         _check(lib().b200_selftest_wait_timeout(self._h, stream), "selftest_wait_timeout")
 
     def op(self, name, *args):
-        """Calls any other entry point by name (the elementwise / movement / reduction set).  An open
-        context has the native form of this in its place."""
-        _call_ctypes(self._h, name, *args)
+        """Calls any other entry point by name (the elementwise / movement / reduction set).  Once the
+        library is loaded the native form of this stands in its place."""
+        _check(getattr(lib(), name)(self._h, *args), name)
 
     def gemm(self, mode, trans_a, trans_b, A, B, C, m, n, k, groups=1, red=1,
              a_gs=0, a_rs=0, b_gs=0, b_rs=0, c_gs=0, accumulate=False, force_path=0, stream=None):

@@ -1,6 +1,8 @@
 """The native call path of ``Context.op`` (primitiv_b200/binding/native.cc) without a GPU: which calls it
 takes, what it hands to the ctypes path, and how a failure code comes back."""
 import ctypes
+import gc
+import weakref
 
 import pytest
 
@@ -47,3 +49,74 @@ def test_wrapped_names_are_entry_points_and_errors_are_raised():
             with pytest.raises(pb.B200Error) as e:
                 op(name, *[0.0 if t is ctypes.c_float else 0 for t in argtypes[1:]])
             assert e.value.code == INVALID
+
+
+@pytest.fixture()
+def destroyed(monkeypatch):
+    """Contexts without a GPU: creation hands out an address that nothing follows, destruction notes it."""
+    real, gone = pb.lib(), []
+
+    class Library:
+        def b200_ctx_create(self, device, out):
+            out._obj.value = 4096
+            return 0
+
+        def b200_ctx_destroy(self, h):
+            gone.append(h.value)
+
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+    stand_in = Library()
+    monkeypatch.setattr(capi, "lib", lambda: stand_in)
+    yield gone
+    gc.collect()
+
+
+FILL = ("b200_fill", 0, 256, 4, 0.5, None)
+
+
+def test_a_kept_op_keeps_its_context_alive(destroyed):
+    c = pb.Context(0)
+    op, alive = c.op, weakref.ref(c)
+    del c
+    gc.collect()
+    assert alive() is not None and not destroyed
+    del op
+    assert alive() is None and destroyed == [4096]   # at once: no cycle holds a context until the next collection
+
+
+def test_a_closed_context_has_a_null_pointer(destroyed):
+    c = pb.Context(0)
+    op = c.op
+    c.close()
+    c.close()
+    assert destroyed == [4096]
+    for call in (op, c.op):
+        with pytest.raises(pb.B200Error) as e:
+            call(*FILL)
+        assert e.value.code == INVALID
+
+
+def test_a_subclass_can_put_its_own_op_in_place(destroyed):
+    class Other(pb.Context):
+        def op(self, name, *args):
+            raise AssertionError("looked up, not called")
+
+    assert Other(0).op.__func__ is Other.op
+
+
+def test_an_object_without_an_address_goes_to_the_fallback():
+    pb.lib()
+    from primitiv_b200 import _native
+    seen = []
+
+    class Other:
+        op = _native.caller(None, lambda *a: seen.append(a), None)
+
+    o = Other()
+    o.op(*FILL)
+    for address in (None, "0", 2 ** 70):
+        o._address = address
+        o.op(*FILL)
+    assert seen == [(o,) + FILL] * 4
