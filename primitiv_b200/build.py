@@ -19,7 +19,8 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(PKG, "libprimitiv_b200.so")
 BINDING = os.path.join(PKG, "binding", "native.cc")
-NATIVE = os.path.join(PKG, "_native.so")   # CPython module over the library
+# CPython module over the library.  The name carries the interpreter's tag, so that another interpreter does not import it.
+NATIVE = os.path.join(PKG, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -43,6 +44,25 @@ def _stale(out, deps):
         return True
     t = os.path.getmtime(out)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _build_native(force):
+    untagged = os.path.join(PKG, "_native.so")
+    if os.path.exists(untagged):
+        os.remove(untagged)   # of an earlier build, for whichever interpreter
+    include = sysconfig.get_paths()["include"]
+    if not os.path.exists(os.path.join(include, "Python.h")):
+        sys.stderr.write("note: no Python.h in %s; calls go through ctypes (5.3 us instead of 2.7)\n" % include)
+        return
+    headers = [os.path.join(os.path.dirname(PKG), "include", f) for f in ("primitiv_b200.h", "primitiv_b200_ops.h")]
+    if not force and not _stale(NATIVE, [BINDING, os.path.abspath(__file__)] + headers):
+        return
+    cmd = ["g++", "-O3", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall", "-I" + include, BINDING, "-o", NATIVE,
+           "-L" + PKG, "-lprimitiv_b200", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed: " + BINDING)
 
 
 def build(verbose=False, force=False, dev_knobs=False):
@@ -87,15 +107,7 @@ def build(verbose=False, force=False, dev_knobs=False):
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
-    headers = [os.path.join(os.path.dirname(PKG), "include", f) for f in ("primitiv_b200.h", "primitiv_b200_ops.h")]
-    if force or _stale(NATIVE, [BINDING, os.path.abspath(__file__)] + headers):
-        cmd = ["g++", "-O3", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall",
-               "-I" + sysconfig.get_paths()["include"], BINDING, "-o", NATIVE, "-L" + PKG, "-lprimitiv_b200",
-               "-Wl,-rpath,$ORIGIN"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            sys.stderr.write(r.stdout + r.stderr)
-            raise RuntimeError("g++ failed: " + BINDING)
+    _build_native(force)
     with open(stamp, "w") as f:
         f.write(" ".join(flags))
     return LIB

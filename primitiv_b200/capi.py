@@ -6,7 +6,8 @@ no compute of its own.
 
 ``lib()`` is the library through ctypes.  The entry points that a training step calls
 thousands of times go through ``_native`` (binding/native.cc) instead, which takes plain
-numbers and None only; ``Context.op`` tries it first.
+numbers and None only; ``Context.op`` tries it first, and does without where it is not built for
+this interpreter.
 """
 import ctypes
 import os
@@ -132,9 +133,9 @@ def lib():
             fn.argtypes = args
         try:
             from . import _native
-        except ImportError as e:
-            raise ImportError("primitiv_b200/_native.so is not built (run `python -m primitiv_b200.build`): %s" % e) from e
-        Context.op = _native.caller(None, Context.op, _check)
+            Context.op = _native.caller(None, Context.op, _check)
+        except ImportError:
+            pass   # built without Python's headers, or for another interpreter: the same calls through ctypes
         _LIB = handle
     return _LIB
 
@@ -290,8 +291,8 @@ class Context:
         _check(lib().b200_selftest_wait_timeout(self._h, stream), "selftest_wait_timeout")
 
     def op(self, name, *args):
-        """Calls any other entry point by name (the elementwise / movement / reduction set).  Once the
-        library is loaded the native form of this stands in its place."""
+        """Calls any other entry point by name (the elementwise / movement / reduction set).  Where
+        there is a native form of this, it stands in its place once the library is loaded."""
         _check(getattr(lib(), name)(self._h, *args), name)
 
     def gemm(self, mode, trans_a, trans_b, A, B, C, m, n, k, groups=1, red=1,

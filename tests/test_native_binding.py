@@ -2,6 +2,9 @@
 takes, what it hands to the ctypes path, and how a failure code comes back."""
 import ctypes
 import gc
+import subprocess
+import sys
+import sysconfig
 import weakref
 
 import pytest
@@ -120,3 +123,27 @@ def test_an_object_without_an_address_goes_to_the_fallback():
         o._address = address
         o.op(*FILL)
     assert seen == [(o,) + FILL] * 4
+
+
+def test_the_native_form_is_this_interpreters_own():
+    pb.lib()
+    from primitiv_b200 import _native
+    assert _native.__file__.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def test_calls_go_without_the_native_form():
+    """Where there is none (no Python headers, another interpreter) every call goes through ctypes."""
+    code = """if True:
+        import sys
+        sys.modules["primitiv_b200._native"] = None     # what an import of it then finds
+        import primitiv_b200 as pb
+        pb.lib()
+        c = pb.Context.__new__(pb.Context)
+        c._h = None
+        try:
+            c.matmul_fw(0, 256, 256, 256, 1, 1, 1, 1, 1)
+        except pb.B200Error as e:
+            print(e.code)
+    """
+    r = subprocess.run([sys.executable, "-c", code], cwd=capi._PKG + "/..", capture_output=True, text=True)
+    assert r.stdout.split() == [str(INVALID)], r.stdout + r.stderr
