@@ -275,24 +275,55 @@ __device__ __forceinline__ float4 ld_cluster(uint32_t addr, uint32_t rank) {
 }
 
 // An infinite operand makes x - hi a nan, or meets the zero it left of another one.  Products that are the CUDA
-// cores' by their numerics (has_fp32_sums) sum an element that is not finite again as those do.
+// cores' by their numerics (has_fp32_sums) sum elements that are not finite again in plain fp32: four rows i .. i + 3 of
+// column j, by a whole warp with its lanes side by side in k (K-major A), or by each lane for itself, whose
+// neighbours have the rows beside its own.  Bound by latency, hence many loads in flight: of nothing but nans 64 x 8 x 65536
+// takes 5.8 ms (3.6 with K-major A) and 1000 x 12 x 20000 2.9; one element and one load at a time it was 41 (14.7) and 26,
+// on the CUDA cores 4.9 (5.5) and 1.9.
 template <bool KA, bool KB>
-__device__ __noinline__ float plain_sum(const MmaParams &p, uint32_t g, uint32_t i, uint32_t j) {
-  float v = 0.f;
+__device__ __noinline__ float4 plain_sums(const MmaParams &p, uint32_t g, uint32_t i, uint32_t j) {
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  unsigned long long row[4];
+#pragma unroll
+  for (uint32_t e = 0; e < 4u; ++e) row[e] = (i + e < p.m ? i + e : p.m - 1u) * (KA ? p.lda : 1ull);
   for (uint32_t r = 0; r < p.kt / p.kb; ++r) {
-    const float *a = static_cast<const float *>(p.A) + g * p.a_gs + r * p.a_rs + i * (KA ? p.lda : 1ull);
+    const float *a = static_cast<const float *>(p.A) + g * p.a_gs + r * p.a_rs;
     const float *b = static_cast<const float *>(p.B) + g * p.b_gs + r * p.b_rs + j * (KB ? p.ldb : 1ull);
-    for (uint32_t k = 0; k < p.k; ++k) v = fmaf(a[k * (KA ? 1ull : p.lda)], b[k * (KB ? 1ull : p.ldb)], v);
+#pragma unroll KA ? 8 : 16
+    for (uint32_t k = KA ? threadIdx.x & 31u : 0u; k < p.k; k += KA ? 32u : 1u) {
+      const float y = b[k * (KB ? 1ull : p.ldb)];
+#pragma unroll
+      for (uint32_t e = 0; e < 4u; ++e) v[e] = fmaf(a[row[e] + k * (KA ? 1ull : p.lda)], y, v[e]);
+    }
   }
-  return v;
+  if constexpr (KA) {
+#pragma unroll
+    for (uint32_t o = 16; o > 0u; o >>= 1) {
+#pragma unroll
+      for (uint32_t e = 0; e < 4u; ++e) v[e] += __shfl_xor_sync(0xffffffffu, v[e], o);
+    }
+  }
+  return make_float4(v[0], v[1], v[2], v[3]);
 }
+// Called by whole warps; `inside`: this lane's v is of the result.
 template <bool KA, bool KB>
-__device__ __forceinline__ void mend(float4 &v, const MmaParams &p, uint32_t g, uint32_t i, uint32_t j) {
-  if (!p.mend || fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) <= 3e38f) return;
-  if (!(fabsf(v.x) <= 3e38f)) v.x = plain_sum<KA, KB>(p, g, i, j);
-  if (!(fabsf(v.y) <= 3e38f) && i + 1u < p.m) v.y = plain_sum<KA, KB>(p, g, i + 1u, j);
-  if (!(fabsf(v.z) <= 3e38f) && i + 2u < p.m) v.z = plain_sum<KA, KB>(p, g, i + 2u, j);
-  if (!(fabsf(v.w) <= 3e38f) && i + 3u < p.m) v.w = plain_sum<KA, KB>(p, g, i + 3u, j);
+__device__ __forceinline__ void mend(float4 &v, bool inside, const MmaParams &p, uint32_t g, uint32_t i, uint32_t j) {
+  const bool odd = inside && !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) <= 3e38f);
+  float4 w = v;
+  if constexpr (KA) {
+#pragma unroll 1
+    for (uint32_t left = __ballot_sync(0xffffffffu, odd); left != 0u; left &= left - 1u) {
+      const int lane = __ffs(left) - 1;
+      const float4 sums = plain_sums<KA, KB>(p, g, __shfl_sync(0xffffffffu, i, lane), __shfl_sync(0xffffffffu, j, lane));
+      if ((threadIdx.x & 31u) == static_cast<uint32_t>(lane)) w = sums;
+    }
+  } else {
+    if (odd) w = plain_sums<KA, KB>(p, g, i, j);
+  }
+  if (!(fabsf(v.x) <= 3e38f)) v.x = w.x;
+  if (!(fabsf(v.y) <= 3e38f)) v.y = w.y;
+  if (!(fabsf(v.z) <= 3e38f)) v.z = w.z;
+  if (!(fabsf(v.w) <= 3e38f)) v.w = w.w;
 }
 
 template <int KIND, int BM, int BN, int WM, int WN, int STAGES>
@@ -497,7 +528,7 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
   if (p.splits > 1u) cluster_barrier();
   else __syncthreads();
 
-  // Every CTA of the cluster finishes its share of the tile.
+  // Every CTA of the cluster finishes its share of the tile, in rounds of whole warps (32 divides the tile's quads).
   T *C = static_cast<T *>(p.C) + g * p.c_gs;
   const bool along_m = p.c_m == 1u;
   if (along_m) {
@@ -507,7 +538,8 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
     for (uint32_t q = threadIdx.x + rank * NT; q < kQuads * BN; q += NT * p.splits) {
       const uint32_t nn = q / kQuads, mm = (q % kQuads) * 4u;
       const uint32_t gm = m0 + mm, gn = n0 + nn;
-      if (gn >= p.n || gm >= p.m) continue;
+      const bool inside = gn < p.n && gm < p.m;
+      if (!inside && (KIND != kMmaFp32 || !p.mend)) continue;   // (warps stay whole where elements may be summed again)
       const uint32_t at = base + (nn * Tile::kPitch + mm) * 4u;
       float4 v;
       if (p.splits > 1u) {
@@ -519,7 +551,10 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
       } else {
         v = *reinterpret_cast<const float4 *>(out + nn * Tile::kPitch + mm);
       }
-      if constexpr (KIND == kMmaFp32) mend<KA, KB>(v, p, g, gm, gn);
+      if constexpr (KIND == kMmaFp32) {
+        if (p.mend) mend<KA, KB>(v, inside, p, g, gm, gn);
+        if (!inside) continue;
+      }
       T *c = C + gm + gn * p.c_n;
       const bool whole = gm + 4u <= p.m && (reinterpret_cast<unsigned long long>(c) & (4u * kES - 1u)) == 0;
       if (whole) {
@@ -551,7 +586,8 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
     for (uint32_t q = threadIdx.x + rank * NT; q < (BM / 4) * BN; q += NT * p.splits) {
       const uint32_t nn = q % BN, mm = (q / BN) * 4u;
       const uint32_t gm = m0 + mm, gn = n0 + nn;
-      if (gn >= p.n || gm >= p.m) continue;
+      const bool inside = gn < p.n && gm < p.m;
+      if (!inside && (KIND != kMmaFp32 || !p.mend)) continue;   // (warps stay whole where elements may be summed again)
       const uint32_t at = base + (nn * Tile::kPitch + mm) * 4u;
       float4 v;
       if (p.splits > 1u) {
@@ -563,7 +599,10 @@ __global__ void __launch_bounds__(MmaTile<KIND, BM, BN, WM, WN, STAGES>::kThread
       } else {
         v = *reinterpret_cast<const float4 *>(out + nn * Tile::kPitch + mm);
       }
-      if constexpr (KIND == kMmaFp32) mend<KA, KB>(v, p, g, gm, gn);
+      if constexpr (KIND == kMmaFp32) {
+        if (p.mend) mend<KA, KB>(v, inside, p, g, gm, gn);
+        if (!inside) continue;
+      }
       T *c = C + gm * p.c_m + gn;
       const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
