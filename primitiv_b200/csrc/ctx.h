@@ -126,6 +126,7 @@ struct PlaneCache {
   std::size_t bytes = 0, cap = 0;   // cap == 0: not enabled by the caller
   int scope = 0;                    // > 0 inside an entry point that shares planes between its products
   std::uint64_t clock = 0, hits = 0, misses = 0;
+  std::uint64_t settled = 0;        // entries stamped later belong to the product that is being prepared: not to be evicted
   bool active() const { return cap != 0 || scope > 0; }
 };
 

@@ -846,6 +846,7 @@ double pack_us(const b200_ctx *ctx, const OperandView &v, int mode, bool is_b, u
 int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fixed_scratch,
                 uint64_t fixed_elems) {
   if (!gemm_tc_eligible(ctx, g)) return B200_ERR_INVALID_ARG;
+  ctx->planes.settled = ctx->planes.clock;
   const bool half_store = g.mode == B200_MODE_FP16;        // operands and C are half in memory
   const bool split16 = g.mode == B200_MODE_FP32_3XFP16;    // fp32 in memory, two half planes per operand
   const bool f16 = half_store || split16;                  // what the tensor core is fed: kind::f16

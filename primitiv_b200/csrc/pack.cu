@@ -912,10 +912,14 @@ int flat_planes(b200_ctx *ctx, cudaStream_t stream, OperandView &v, PlaneKind ki
     *owned_block = block;
     return B200_OK;
   }
-  while (pc.bytes + block_bytes > cap && !pc.entries.empty()) {   // least recently used first
-    std::size_t oldest = 0;
-    for (std::size_t i = 1; i < pc.entries.size(); ++i)
-      if (pc.entries[i].stamp < pc.entries[oldest].stamp) oldest = i;
+  while (pc.bytes + block_bytes > cap) {   // least recently used first, but for the other operand of this product
+    std::size_t oldest = pc.entries.size();
+    for (std::size_t i = 0; i < pc.entries.size(); ++i)
+      if (pc.entries[i].stamp <= pc.settled && (oldest == pc.entries.size() || pc.entries[i].stamp < pc.entries[oldest].stamp)) oldest = i;
+    if (oldest == pc.entries.size()) {
+      *owned_block = block;
+      return B200_OK;
+    }
     void *old = pc.entries[oldest].block;
     pc.bytes -= pc.entries[oldest].block_bytes;
     pc.entries[oldest] = pc.entries.back();

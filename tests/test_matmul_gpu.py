@@ -237,6 +237,31 @@ def test_operand_cache_forgets_what_is_written(ctx):
         ctx.set_path_policy(0)
 
 
+@pytest.mark.parametrize("n", [256, 250])
+@pytest.mark.parametrize("size", [(256, 4096), (128, 8192), (384, 2048)], ids=lambda s: "%dx%d" % s)
+def test_operand_cache_never_evicts_the_other_operand(ctx, size, n):
+    """A cap that holds either operand's planes but not both, on products whose contraction is split: the second
+    operand's planes must not take the first's block away before the launch (the scratch of the slices would get it)."""
+    m, k = size
+    rng = np.random.default_rng(47)
+    a, b = (rng.uniform(-1, 1, s).astype(np.float32) for s in (m * k, k * n))
+    da, db, y = _cuda(a), _cuda(b), torch.empty(m * n, device="cuda")
+    want = ol.fw_f64(a, b, m, k, n, 1, 1)
+    planes = 8 * max(m, n + 8) * k
+    ctx.set_path_policy(2)
+    try:
+        for cap in (planes + 4096, planes * 3 // 2):
+            ctx.operand_cache_enable(cap)
+            for _ in range(3):
+                ctx.matmul_fw(pb.MODE_FP32_3XTF32, da.data_ptr(), db.data_ptr(), y.data_ptr(), m, k, n, 1, 1)
+                assert ol.rel_err(y.cpu().numpy(), want) <= 1e-5
+                assert ctx.operand_cache_stats()["bytes"] <= cap
+            ctx.operand_cache_enable(0)
+    finally:
+        ctx.operand_cache_enable(0)
+        ctx.set_path_policy(0)
+
+
 def test_backward_call_packs_the_upstream_gradient_once(ctx):
     """Without the cache: inside one b200_matmul_bw call gy still serves both products from one set of
     planes (one hit), and nothing is kept afterwards."""
