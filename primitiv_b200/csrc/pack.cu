@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256) row_max_mnmajor_vec_kernel(const float *_
                                                                   unsigned long long src_bs, uint32_t nbatch, int shared,
                                                                   uint32_t k_slice) {
   pdl_enter();
-  __shared__ float buf[8][132];
+  __shared__ __align__(16) float buf[8][132];
   const uint32_t tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
   const uint32_t tiles = (mn + 127u) / 128u;
   const unsigned long long total = static_cast<unsigned long long>(tiles) * nbatch;
