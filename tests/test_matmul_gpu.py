@@ -262,6 +262,61 @@ def test_operand_cache_never_evicts_the_other_operand(ctx, size, n):
         ctx.set_path_policy(0)
 
 
+def test_padded_planes_go_stale_as_the_others_do(ctx):
+    """Ragged fp32 arrays, whose padded planes are kept across calls too: a second use finds them, and they are
+    forgotten when the caller says so, when a product overwrites the array, when its block returns to the pool,
+    and, least recently used first, when the cap is reached."""
+    n = 251
+    rng = np.random.default_rng(53)
+    a, b, c, a2 = (rng.uniform(-1, 1, n * n).astype(np.float32) for _ in range(4))
+    da, db, dc = _cuda(a), _cuda(b), _cuda(c)
+    y, z = torch.empty(n * n, device="cuda"), torch.empty(n * n, device="cuda")
+    M = pb.MODE_FP32_3XTF32
+    fw = lambda p, q, r: ctx.matmul_fw(M, p.data_ptr(), q.data_ptr(), r.data_ptr(), n, n, n, 1, 1)
+    ref = lambda p, q: ol.fw_f64(p, q, n, n, n, 1, 1)
+    counts = lambda: (lambda s: (s["hits"], s["misses"], s["entries"]))(ctx.operand_cache_stats())
+    ctx.set_path_policy(2)
+    ctx.operand_cache_enable(1 << 30)
+    try:
+        h, m, _ = counts()
+        fw(da, db, y)
+        assert counts() == (h, m + 2, 2)
+        fw(da, db, y)
+        assert counts() == (h + 2, m + 2, 2)
+        fw(y, dc, z)                                    # planes of y and c
+        assert counts() == (h + 2, m + 4, 4)
+        da.copy_(_cuda(a2))
+        ctx.operand_cache_invalidate(da.data_ptr(), da.numel() * 4)
+        assert counts()[2] == 3
+        fw(da, db, y)                                   # packs a again, and y's planes go: it is overwritten
+        assert counts() == (h + 3, m + 5, 3)
+        fw(y, dc, z)
+        y2 = ref(a2, b)
+        assert ol.rel_err(y.cpu().numpy(), y2) <= 1e-5
+        assert ol.rel_err(z.cpu().numpy(), ref(y2.astype(np.float32), c)) <= 1e-5
+        p1, _ = ctx.pool_alloc(n * n * 4)
+        ctx.op("b200_upload", M, a.ctypes.data, p1, n * n, None)
+        ctx.matmul_fw(M, p1, db.data_ptr(), y.data_ptr(), n, n, n, 1, 1)
+        before = counts()[2]
+        ctx.pool_free(p1)
+        assert counts()[2] == before - 1
+        ctx.operand_cache_enable(0)
+        ctx.operand_cache_enable(3 * 8 * n * 256)       # three sets of planes
+        fw(da, db, y)
+        fw(da, dc, z)                                   # a, c newer than b
+        _, m, entries = counts()
+        assert entries == 3
+        fw(dc, db, z)                                   # both found
+        fw(z, dc, y)                                    # z evicts a, the oldest
+        assert counts()[1:] == (m + 1, 3)
+        fw(da, dc, y)
+        assert counts()[1] == m + 2
+        assert ol.rel_err(y.cpu().numpy(), ref(a2, c)) <= 1e-5
+    finally:
+        ctx.operand_cache_enable(0)
+        ctx.set_path_policy(0)
+
+
 def test_backward_call_packs_the_upstream_gradient_once(ctx):
     """Without the cache: inside one b200_matmul_bw call gy still serves both products from one set of
     planes (one hit), and nothing is kept afterwards."""
