@@ -81,6 +81,7 @@ int b200_ctx_create(int device_id, b200_ctx **out) {
   // a block that returns to the pool takes the planes packed from its contents with it
   ctx->pool.on_free = [ctx](const void *p, std::size_t bytes) { b200::plane_cache_drop_range(ctx, p, bytes); };
   ctx->pool.before_release = [ctx]() { b200::queue_drain(ctx); };
+  ctx->pool.on_exhausted = [ctx]() { return b200::plane_cache_make_room(ctx); };
   ctx->staging.before_copy = [ctx]() { b200::queue_drain(ctx); };
   void *fn = nullptr;
   cudaDriverEntryPointQueryResult qres;
@@ -344,7 +345,10 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   // Planes that happen to be held may only decide where both kernels give the same bits: the same call on the same operands
   // has to give the same twice.
   if (one_order) tc = b200::gemm_tc_estimate(ctx, g, true);
-  return direct < tc ? b200::gemm_direct(ctx, g, s) : b200::gemm_tc(ctx, g, s);
+  if (direct < tc) return b200::gemm_direct(ctx, g, s);
+  const int rc = b200::gemm_tc(ctx, g, s);
+  // Ragged halves had no need of scratch before their lines were padded, and have a kernel that needs none.
+  return rc == B200_ERR_OUT_OF_MEMORY && mode == B200_MODE_FP16 ? b200::gemm_mma(ctx, g, s) : rc;
 }
 
 int b200_gemm_3xtf32_noalloc(b200_ctx *ctx, int trans_a, int trans_b, const void *A, const void *B,

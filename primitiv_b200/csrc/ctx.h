@@ -29,6 +29,7 @@ class Pool {
   int alloc(std::size_t bytes, void **ptr, std::size_t *allocated);
   int free(void *ptr);
   void release_cached();
+  bool has(std::size_t bytes) const;   // alloc(bytes) would not ask the driver
   void stats(std::uint64_t out[4]) const;
   // Test hook: a soft capacity (0 = none).  Requests that would push
   // in-use + cached bytes past it behave exactly like a failed cudaMalloc.
@@ -47,6 +48,9 @@ class Pool {
   // Called before cached blocks are handed back to the driver: the context uses it to issue
   // launches that are still waiting in its launch queue and may read those blocks.
   std::function<void()> before_release;
+  // Called when memory has run out even so, before an allocation fails: returns blocks to the pool that are only held to save
+  // work (cached operand planes), or false if there are none.
+  std::function<bool()> on_exhausted;
 
  private:
   std::map<std::size_t, std::vector<void *>> cached_;
@@ -126,7 +130,12 @@ struct PlaneCache {
   std::size_t bytes = 0, cap = 0;   // cap == 0: not enabled by the caller
   int scope = 0;                    // > 0 inside an entry point that shares planes between its products
   std::uint64_t clock = 0, hits = 0, misses = 0;
-  std::uint64_t settled = 0;        // entries stamped later belong to the product that is being prepared: not to be evicted
+  std::uint64_t settled = ~0ull;    // entries stamped later belong to the product that is being prepared: not to be evicted
+  struct Use {                      // brackets that product, from its first look at the planes to its launch
+    PlaneCache &planes;
+    explicit Use(PlaneCache &p) : planes(p) { p.settled = p.clock; }
+    ~Use() { planes.settled = ~0ull; }
+  };
   bool active() const { return cap != 0 || scope > 0; }
 };
 
@@ -269,6 +278,11 @@ int gemm_3xtf32_noalloc(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream);
 // [ptr, ptr + bytes) (everything when ptr is null) and returns its block to the pool.
 void plane_cache_drop_range(b200_ctx *ctx, const void *ptr, std::size_t bytes);
 void plane_cache_drop_call_only(b200_ctx *ctx);
+// Returns the blocks of all planes that no product in preparation uses to the pool; false: there were none.
+bool plane_cache_make_room(b200_ctx *ctx);
+// Scratch from the pool that there is a way without: none, either, where a graph is being captured and the pool would have
+// to ask the driver, which ends the capture.
+int optional_scratch_alloc(b200_ctx *ctx, cudaStream_t stream, std::size_t bytes, void **ptr);
 // Brackets an entry point that hands the same operand to several products.
 struct PlaneScope {
   b200_ctx *ctx;

@@ -846,7 +846,7 @@ double pack_us(const b200_ctx *ctx, const OperandView &v, int mode, bool is_b, u
 int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fixed_scratch,
                 uint64_t fixed_elems) {
   if (!gemm_tc_eligible(ctx, g)) return B200_ERR_INVALID_ARG;
-  ctx->planes.settled = ctx->planes.clock;
+  const PlaneCache::Use own_planes(ctx->planes);
   const bool half_store = g.mode == B200_MODE_FP16;        // operands and C are half in memory
   const bool split16 = g.mode == B200_MODE_FP32_3XFP16;    // fp32 in memory, two half planes per operand
   const bool f16 = half_store || split16;                  // what the tensor core is fed: kind::f16
@@ -909,14 +909,15 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   const void *a_src[2] = {g.A, nullptr}, *b_src[2] = {g.B, nullptr};
   const void *a_mix[3] = {nullptr, nullptr, nullptr}, *b_mix[3] = {nullptr, nullptr, nullptr};
   void *flat_blocks[2] = {nullptr, nullptr};  // flat planes that the cache did not take: freed after the launch
-  void *scratch = nullptr;
+  void *scratch = nullptr, *partial = nullptr;
   auto release = [&]() {   // stream-ordered reuse: later work queues behind this product
     if (scratch) ctx->pool.free(scratch);
+    if (partial) ctx->pool.free(partial);
     for (void *&blk : flat_blocks) {
       if (blk) ctx->pool.free(blk);
       blk = nullptr;
     }
-    scratch = nullptr;
+    scratch = partial = nullptr;
   };
   // kind 4 bookkeeping: the plane pointers of each operand and whether they are flat copies
   bool a_flat = false, b_flat = false;
@@ -979,12 +980,10 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
       } else if (o == 1 && b_hybrid) {
         vb8 = vb;   // the caller's layout: what the cached planes repeat
         const void *cached_planes[3];
-        void *unused = nullptr;
-        const int rc = flat_planes(ctx, stream, vb8, kPlanesMix, cached_planes, &unused);   // a cache hit: nothing is packed
-        if (rc != B200_OK || unused) {
-          if (unused) ctx->pool.free(unused);
+        const int rc = flat_planes(ctx, stream, vb8, kPlanesMix, cached_planes, &flat_blocks[o]);   // a cache hit, unless the scratch took their place
+        if (rc != B200_OK) {
           release();
-          return rc != B200_OK ? rc : B200_ERR_INVALID_ARG;
+          return rc;
         }
         pack_mix(ctx, stream, vb, cursor, lay[o], outs[o], /*hi_only=*/true);
         cursor += lay[o].hi_elems;
@@ -1100,11 +1099,20 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   p.kblocks = (g.k + p.bk * p.subs - 1) / (p.bk * p.subs);  // pipeline-stage iterations along k
   // Split-K: slices of k go to CTAs (or pairs) that the tiles alone would leave idle, and splitk_reduce_kernel adds them up.
   uint32_t splits = 1;
-  void *partial = nullptr;
   if (tile.splits > 1u && !wide) {   // (the wide epilogue stores halves only)
     const uint32_t per = (p.kblocks + tile.splits - 1u) / tile.splits;
     splits = (p.kblocks + per - 1u) / per;  // no empty slices
-    p.kblocks = per;
+    // A product of one pass may need no other scratch: without memory for the slices it is not split.
+    const size_t bytes = static_cast<size_t>(g.m) * g.n * g.groups * splits * sizeof(float);
+    const int rc = splits == 1u ? B200_OK : passes == 1 ? optional_scratch_alloc(ctx, stream, bytes, &partial) : ctx->pool.alloc(bytes, &partial, nullptr);
+    if (rc == B200_ERR_OUT_OF_MEMORY && passes == 1) {
+      splits = 1;
+    } else if (rc != B200_OK) {
+      release();
+      return rc;
+    } else {
+      p.kblocks = per;
+    }
   }
   p.splits = splits;
   p.groups = g.groups * splits;
@@ -1235,14 +1243,8 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
   p.C = g.C;
   p.c_gs = g.c_gs;
   if (splits > 1) {
-    const uint64_t mn = static_cast<uint64_t>(g.m) * g.n;
-    const int arc = ctx->pool.alloc(mn * g.groups * splits * sizeof(float), &partial, nullptr);
-    if (arc != B200_OK) {
-      release();
-      return arc;
-    }
     p.C = partial;
-    p.c_gs = mn;
+    p.c_gs = static_cast<uint64_t>(g.m) * g.n;
     p.accumulate = 0u;
     p.out_half = 0u;
   }
@@ -1366,7 +1368,6 @@ int gemm_tc_run(b200_ctx *ctx, const GemmArgs &g, cudaStream_t stream, float *fi
       rc = static_cast<int>(cudaGetLastError());
     }
   }
-  if (partial) ctx->pool.free(partial);
   release();
   return rc;
 }

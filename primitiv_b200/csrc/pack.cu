@@ -802,6 +802,34 @@ void plane_cache_drop_call_only(b200_ctx *ctx) {
   for (void *b : blocks) ctx->pool.free(b);
 }
 
+bool plane_cache_make_room(b200_ctx *ctx) {
+  PlaneCache &pc = ctx->planes;
+  std::vector<void *> blocks;
+  for (std::size_t i = 0; i < pc.entries.size();) {
+    if (pc.entries[i].stamp <= pc.settled) {
+      blocks.push_back(pc.entries[i].block);
+      pc.bytes -= pc.entries[i].block_bytes;
+      pc.entries[i] = pc.entries.back();
+      pc.entries.pop_back();
+    } else {
+      ++i;
+    }
+  }
+  for (void *b : blocks) ctx->pool.free(b);
+  return !blocks.empty();
+}
+
+int optional_scratch_alloc(b200_ctx *ctx, cudaStream_t stream, std::size_t bytes, void **ptr) {
+  if (!ctx->pool.has(bytes)) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
+      cudaGetLastError();
+      return B200_ERR_OUT_OF_MEMORY;
+    }
+  }
+  return ctx->pool.alloc(bytes, ptr, nullptr);
+}
+
 namespace {
 
 // What identifies a set of planes besides its kind: the array, and its line length where lines are padded.
@@ -876,7 +904,8 @@ int flat_planes(b200_ctx *ctx, cudaStream_t stream, OperandView &v, PlaneKind ki
     ++pc.misses;
   }
   void *block = nullptr;
-  const int rc = ctx->pool.alloc(block_bytes, &block, nullptr);
+  // (products of halves have a kernel that needs no padded lines)
+  const int rc = kind == kPlanesHalf ? optional_scratch_alloc(ctx, stream, block_bytes, &block) : ctx->pool.alloc(block_bytes, &block, nullptr);
   if (rc != B200_OK) return rc;
   planes_of(block);
   void *p0 = block, *p1 = const_cast<void *>(planes_out[1]), *p2 = const_cast<void *>(planes_out[2]);

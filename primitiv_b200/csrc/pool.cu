@@ -78,6 +78,10 @@ int Pool::alloc(std::size_t bytes, void **ptr, std::size_t *allocated) {
       release_cached();
       rc = raw_alloc(cls, ptr);
     }
+    if (rc == B200_ERR_OUT_OF_MEMORY && on_exhausted && on_exhausted()) {
+      release_cached();
+      rc = raw_alloc(cls, ptr);
+    }
     if (rc != B200_OK) return rc;
   }
   in_use_[*ptr] = cls;
@@ -97,6 +101,11 @@ int Pool::free(void *ptr) {
   cached_[cls].push_back(ptr);
   bytes_cached_ += cls;
   return B200_OK;
+}
+
+bool Pool::has(std::size_t bytes) const {
+  auto it = cached_.find(size_class(bytes ? bytes : 1));
+  return it != cached_.end() && !it->second.empty();
 }
 
 void Pool::release_cached() {

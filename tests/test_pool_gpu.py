@@ -176,3 +176,87 @@ def test_large_uploads_arrive_intact(own_ctx, n, half):
         c.op("b200_download", m, ptr, got.ctypes.data, want.size, None)
         assert np.array_equal(got, want)
         c.pool_free(ptr)
+
+
+def _halves_and_single_pass(c, mode, sizes, check=True):
+    """Forward products with no scratch to be had; returns what to compare after a capture has been replayed."""
+    import torch
+    stream = torch.cuda.current_stream().cuda_stream
+    kind = torch.float16 if mode == pb.MODE_FP16 else torch.float32
+    made = []
+    for m, n, k, groups in sizes:
+        a, b = (torch.randn(groups * s, device="cuda").to(kind) for s in (m * k, k * n))
+        y = torch.empty(groups * m * n, device="cuda", dtype=kind)
+        made.append((a.view(groups, k, m), b.view(groups, n, k), y.view(groups, n, m)))
+        c.gemm(mode, 0, 0, a.data_ptr(), b.data_ptr(), y.data_ptr(), m, n, k, groups, 1, m * k, 0, k * n, 0, m * n, stream=stream)
+    return made
+
+
+def _close(made):
+    for a, b, y in made:
+        want = b.double() @ a.double()
+        assert (y.double() - want).norm() <= 2e-3 * want.norm(), tuple(y.shape)
+
+
+# ragged halves, whose lines would be padded, and single-pass products that read their operands in place but split
+SCRATCHLESS = [(pb.MODE_FP16, [(515, 389, 131, 4), (1021, 765, 131, 2), (130, 200, 5001, 1)]),
+               (pb.MODE_FP16, [(512, 512, 512, 1), (256, 128, 4096, 1)]), (pb.MODE_TF32, [(512, 512, 512, 1), (256, 128, 4096, 1)])]
+
+
+@pytest.mark.parametrize("case", SCRATCHLESS, ids=["ragged_halves", "halves", "tf32"])
+def test_products_that_need_no_scratch_run_without_any(own_ctx, case):
+    own_ctx.pool_set_limit(256)
+    made = _halves_and_single_pass(own_ctx, *case)
+    assert own_ctx.status_poll() == 0
+    _close(made)
+
+
+@pytest.mark.parametrize("case", SCRATCHLESS, ids=["ragged_halves", "halves", "tf32"])
+def test_products_that_need_no_scratch_can_be_captured_first(own_ctx, case):
+    """In a graph, by a context whose pool is still empty: asking the driver for memory would end the capture."""
+    import torch
+    mode, sizes = case
+    graph = torch.cuda.CUDAGraph()
+    stream = torch.cuda.Stream()
+    torch.randn(8, device="cuda").half()
+    with torch.cuda.graph(graph, stream=stream):
+        made = _halves_and_single_pass(own_ctx, mode, sizes)
+    assert own_ctx.pool_stats()["mallocs"] == 0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert own_ctx.status_poll() == 0
+    _close(made)
+
+
+def test_held_planes_make_room_for_an_allocation(own_ctx):
+    """Planes are only kept to save work: what the caller asks the pool for comes first."""
+    import torch
+    n = 1001
+    a, b, y = (torch.randn(n * n, device="cuda") for _ in range(3))
+    own_ctx.operand_cache_enable(1 << 30)
+    own_ctx.set_path_policy(2)
+    own_ctx.pool_set_limit(40 << 20)
+    own_ctx.matmul_fw(pb.MODE_FP32_3XTF32, a.data_ptr(), b.data_ptr(), y.data_ptr(), n, n, n, 1, 1)
+    assert own_ctx.operand_cache_stats()["bytes"] >= 2 * 8 * n * n
+    p, _ = own_ctx.pool_alloc(32 << 20)
+    assert own_ctx.operand_cache_stats()["entries"] == 0
+    own_ctx.pool_free(p)
+    own_ctx.matmul_fw(pb.MODE_FP32_3XTF32, a.data_ptr(), b.data_ptr(), y.data_ptr(), n, n, n, 1, 1)
+    assert own_ctx.status_poll() == 0
+    want = b.view(n, n).double() @ a.view(n, n).double()
+    assert (y.double() - want.flatten()).norm() <= 1e-5 * want.norm()
+
+
+def test_planes_of_earlier_products_make_room(own_ctx):
+    """Both gradients of ragged TF32 operands where the memory holds two padded copies, not three."""
+    import torch
+    n = 1001
+    a, b, gy = (torch.randn(n * n, device="cuda") for _ in range(3))
+    ga, gb = torch.empty_like(a), torch.empty_like(b)
+    own_ctx.set_path_policy(2)
+    own_ctx.pool_set_limit(11 << 20)      # a padded copy takes 4
+    own_ctx.matmul_bw_ex(pb.MODE_TF32, a.data_ptr(), b.data_ptr(), gy.data_ptr(), ga.data_ptr(), gb.data_ptr(), n, n, n, 1, 1, False, False)
+    assert own_ctx.status_poll() == 0
+    a, b, gy = (x.view(n, n).double() for x in (a, b, gy))
+    for got, want in ((ga, b.T @ gy), (gb, gy @ a.T)):
+        assert (got.double() - want.flatten()).norm() <= 2e-3 * want.norm()
