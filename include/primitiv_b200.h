@@ -101,7 +101,8 @@ B200_API int b200_selftest_wait_timeout(b200_ctx *ctx, void *stream);
  * aligned; freed blocks are cached per size class (geometric classes with four
  * steps per octave, so at most ~19% round-up instead of up to 100%); when
  * cudaMalloc fails every cached block is released and the allocation retried once,
- * as the reference pool does. */
+ * as the reference pool does, and once more without the operand planes that are only
+ * held to save work (b200_operand_cache_enable). */
 B200_API int b200_pool_alloc(b200_ctx *ctx, size_t bytes, void **ptr, size_t *allocated_bytes);
 B200_API int b200_pool_free(b200_ctx *ctx, void *ptr);
 B200_API int b200_pool_release_cached(b200_ctx *ctx);
@@ -207,7 +208,8 @@ B200_API int b200_matmul_fw_bw_host(b200_ctx *ctx, int mode,
  * `red` > 1 sums several operand pairs into one C without atomics (the
  * "a batched, b broadcast" gradient that the reference computes with a serial
  * loop of Sgemm calls, matmul.cu:113-123).
- * force_path: 0 = choose; 1 = CUDA-core kernel; 2 = tensor-core kernel (error if ineligible);
+ * force_path: 0 = choose; 1 = CUDA-core kernel; 2 = tensor-core kernel (error if ineligible: two batch
+ * axes on one operand; halves that are neither addressable by TMA nor dense);
  * 3 = the CUDA-core kernels for one tiny extent (m <= 16 or k <= 16) against large ones (error if
  * the shape and layout are not one of theirs); 4 = the mma.sync
  * kernel; 5 = the tcgen05 kernel that loads its operands itself (fp32 modes only); 6 = the CUDA-core
@@ -288,20 +290,22 @@ B200_API int b200_set_dependent_launch(b200_ctx *ctx, int on);
 
 /* ---- operand-plane cache (fp32 mode; no counterpart in the reference) ------------------------------
  * In B200_MODE_FP32_3XTF32 every fp32 operand is split into three planes before the tensor cores see it
- * (4 bytes read and 8 written per element).  A dense operand whose strides are multiples of 8 elements
- * is split "flat": the planes repeat the array's own layout, so the same planes serve every use of the
+ * (4 bytes read and 8 written per element).  A dense operand is split "flat": the planes repeat the
+ * array's own layout, element for element, or with its lines padded to a multiple of 8 elements where
+ * they are not one or the array is not 32-byte aligned; so the same planes serve every use of the
  * array, as either operand of any product.  Inside one call this is automatic (gy feeds both products
  * of b200_matmul_bw; a, b and gy feed two products each in b200_matmul_fw_bw_host).  Across calls the
  * library cannot know whether the array has changed in between, so the caller opts in:
  *
  *   b200_operand_cache_enable(ctx, max_bytes)   keep planes after the call that packed them, least
  *        recently used first out above max_bytes of plane memory (pool memory, twice the operands'
- *        size); 0 switches the cache off and frees it.  Typical use: a training step, where the
- *        backward product receives the very arrays the forward product read.
+ *        size, with padded lines as much more as those are longer: a line of 3 floats takes the room
+ *        of 8); 0 switches the cache off and frees it.  Results do not depend on it.  Typical use: a
+ *        training step, where the backward product receives the very arrays the forward product read.
  *   b200_operand_cache_invalidate(ctx, ptr, bytes)   forget planes packed from any array that overlaps
  *        [ptr, ptr + bytes); ptr == NULL forgets everything.  The caller MUST do this for every
- *        array it (or anything other than the products of this library) writes while the cache is
- *        on.  Two cases are handled inside: the output of b200_gemm / b200_matmul_*, and blocks
+ *        array, ragged ones included, that it (or anything other than the products of this library)
+ *        writes while the cache is on.  Two cases are handled inside: the output of b200_gemm / b200_matmul_*, and blocks
  *        returned through b200_pool_free.  primitiv::devices::B200 calls it from the one place
  *        where it hands out a mutable tensor pointer.
  *   b200_operand_cache_stats   [0] hits, [1] misses, [2] bytes of planes held, [3] entries. */

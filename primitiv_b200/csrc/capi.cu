@@ -329,9 +329,16 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   // would not even fill a k-step of mma.sync (800 x 200 x 10: 3.4 us on the CUDA cores, 4.1 us there).
   // The serial kernel has the CUDA cores' own bits, and up to some 800 terms is faster too (10 x 200 x 800: 8.0 us, 9.7 by
   // mma.sync; 48 x 74 x 491 4.9 and 7.8; 200 x 8 x 1000 9.3 and 6.7).
+  // What TMA cannot address costs the tensor-core kernels narrow copies or a pass that pads lines; the CUDA cores take
+  // any of it as it lies, and are left the sums that are short enough (halves, 88 x 1776 x 7 12 times: 7.3 us, 13.1 with
+  // padded lines; 28 x 338 x 44 4.9 and 8.8 by mma.sync; 51 x 908 x 8, 23 groups of 8: 33 and 65).
+  const bool awkward = mode == B200_MODE_FP16 ? !b200::gemm_tc_reads_in_place(ctx, g) : b200::two_batch_axes(g);
+  const double simt = awkward ? b200::gemm_simt_estimate(ctx, g) : 1e30;
   if (static_cast<double>(m) * n * k * groups * red < 2097152.0) {
     if (static_cast<uint64_t>(k) * red <= 16u) return b200::gemm_simt(ctx, g, s);
-    return b200::gemm_serial_estimate(ctx, g) <= 1.1 * b200::gemm_mma_estimate(ctx, g) ? b200::gemm_serial(ctx, g, s) : b200::gemm_mma(ctx, g, s);
+    const double serial = b200::gemm_serial_estimate(ctx, g), mma = b200::gemm_mma_estimate(ctx, g);
+    if (simt < 0.9 * mma && simt < 0.9 * serial) return b200::gemm_simt(ctx, g, s);
+    return serial <= 1.1 * mma ? b200::gemm_serial(ctx, g, s) : b200::gemm_mma(ctx, g, s);
   }
   // Large products belong to tcgen05 fed by TMA, small fp32 ones to tcgen05 fed by the kernel's own loads, thin and
   // ragged ones to mma.sync: whichever is estimated to take least.
@@ -341,6 +348,7 @@ int b200_gemm(b200_ctx *ctx, int mode, int trans_a, int trans_b, const void *A, 
   // (unless mma.sync is clearly faster the kernels that share one order of summation have the product: 300 x 500 x 333
   // at 12.3 us against 10.6 was within the estimates' error)
   if (one_order) mma *= 1.3;
+  if (simt < 0.9 * mma && simt < 0.9 * tc && simt < 0.9 * direct) return b200::gemm_simt(ctx, g, s);
   if (mma < tc && mma < direct) return b200::gemm_mma(ctx, g, s);
   // Planes that happen to be held may only decide where both kernels give the same bits: the same call on the same operands
   // has to give the same twice.

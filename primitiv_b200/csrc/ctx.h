@@ -231,13 +231,17 @@ struct GemmArgs {
   int accumulate;
 };
 
+// Whether an operand is stepped through along both batch axes.
+inline bool two_batch_axes(const GemmArgs &g) {
+  return g.groups > 1u && g.red > 1u && ((g.a_gs != 0u && g.a_rs != 0u) || (g.b_gs != 0u && g.b_rs != 0u));
+}
+
 // Products with fp32 arithmetic, or as good a split (gemm_mma.cuh), in every mode of fp32 storage, TF32 included: tiny and
 // thin ones, which are bound by latency or by the large operand's bytes, so that it costs next to nothing; and those that step
 // through an operand along both batch axes, which planes cannot follow.
 inline bool has_fp32_sums(const GemmArgs &g) {
   const double macs = static_cast<double>(g.m) * g.n * g.k * g.groups * g.red;
-  if (macs < 2097152.0 || g.n < 16u || (g.m < 32u && macs < 67108864.0)) return true;
-  return g.groups > 1u && g.red > 1u && ((g.a_gs != 0u && g.a_rs != 0u) || (g.b_gs != 0u && g.b_rs != 0u));
+  return macs < 2097152.0 || g.n < 16u || (g.m < 32u && macs < 67108864.0) || two_batch_axes(g);
 }
 
 // CUDA-core path: any shape, any alignment.
@@ -262,6 +266,7 @@ bool gemm_tc_reads_in_place(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_tc_estimate(const b200_ctx *ctx, const GemmArgs &g, bool look);   // look: at the planes that are cached
 double gemm_mma_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_direct_estimate(const b200_ctx *ctx, const GemmArgs &g);
+double gemm_simt_estimate(const b200_ctx *ctx, const GemmArgs &g);
 double gemm_serial_estimate(const b200_ctx *ctx, const GemmArgs &g);
 // The number of slices that every tcgen05 kernel cuts this contraction into; 0: each kernel as it likes.
 uint32_t gemm_fixed_slices(const b200_ctx *ctx, const GemmArgs &g);

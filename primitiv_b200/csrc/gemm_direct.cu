@@ -8,9 +8,9 @@
 // step).  Here eight warps fetch operands with ordinary loads, of any alignment, split each element
 // once, and store the planes where the tensor core reads them; the same warps write the result.
 //
-// A step of 128 x 64 x 32 takes 0.68 us: 48 KB of planes are stored and read again by the tensor core and 24 KB of
-// operands come in, and at 128 bytes per clock that is what shared memory moves.  TMA-fed planes need half of
-// that, so large products stay with gemm_tc.cu.  Measured back to back, planes and reduction included, against
+// A step of 128 x 64 x 32 takes 0.68 us.  48 KB of planes are stored and read again by the tensor core and 24 KB of
+// operands come in: at 128 bytes per clock 960 clocks, 0.49 us, of what shared memory moves; what the other quarter
+// waits for has not been measured.  TMA-fed planes need half of those bytes, so large products stay with gemm_tc.cu.  Measured back to back, planes and reduction included, against
 // gemm_tc.cu: 800 x 200 x 784 14.9 -> 11.2 us, 800 x 784 x 200 12.9 -> 8.5, 512^3 16.0 -> 8.4, 256 x 1024 x 256
 // 12.3 -> 8.2 (gemm_mma.cuh: 17.5, 18.3, 13.0, 9.0).  Slices follow gemm_fixed_slices; tiles of 96 columns let
 // the 5 slices of 800 x 200 run at once (21 clusters, 26 fit; 64 columns make 28), tiles of 32 give unsplit

@@ -208,6 +208,14 @@ int gemm_simt(b200_ctx *ctx, const GemmArgs &a, cudaStream_t s) {
   return launch<float>(ctx, a, s);
 }
 
+// A launch and 1.3 us per step of 16 terms, more where CTAs share an SM: fitted to 220 products of up to 1200 terms, off by 17 %
+// on average.
+double gemm_simt_estimate(const b200_ctx *ctx, const GemmArgs &a) {
+  const double steps = static_cast<double>((a.k + TK - 1) / TK) * a.red;
+  const double waves = static_cast<double>((a.m + TM - 1) / TM) * ((a.n + TN - 1) / TN) * a.groups / ctx->sm_count;
+  return 2.25 + steps * (waves > 1.625 ? 0.8 * waves : 1.3) + (waves > 1.0 ? 0.3 * (waves - 1.0) : 0.0);
+}
+
 // A launch and 0.95 us per slice of k, while four CTAs fit an SM: fitted to 18 products (2.1 us for 64^3, 9.3 for
 // 200 x 8 x 1000, 24.8 for 20 x 30 x 3000).
 double gemm_serial_estimate(const b200_ctx *ctx, const GemmArgs &a) {
